@@ -362,3 +362,27 @@ def test_seq_partition_equivalence():
         for g, t, n in zip(grads, (q, k, v), "qkv"):
             assert torch.allclose(g, t.grad, rtol=1e-2, atol=2e-2), f"{mode} d{n}: {(g - t.grad).abs().max()}"
             t.grad = None
+
+
+@pytest.mark.parametrize("n_seq,k_len", [(17, 4096), (65, 1025)])
+def test_packed_batch_with_more_than_64k_keys_runs_on_tensor_cores(n_seq, k_len):
+    """The 65536-key limit of the tensor-core forward is one sequence's, not the packed batch's: chunks and
+    decode tokens of contexts that together hold more keys stay on it (no fall-back warning) and are right."""
+    import warnings
+    Hq, Hkv, D, bs = 4, 2, 64, 64
+    q_lens = [1 if i % 3 else 33 for i in range(n_seq)]
+    k_lens = [k_len if n % 2 else (k_len // bs) * bs + n for n in q_lens]      # chunks start on a block boundary
+    k_lens = [(kl // bs) * bs + ql if ql > 1 else kl for kl, ql in zip(k_lens, q_lens)]
+    assert sum(k_lens) > 65536
+    pk = dict(block_size=bs, local_blocks=3, vert_stride=5, num_kv_heads=Hkv)
+    cu_q = torch.tensor([0] + list(np.cumsum(q_lens)), dtype=torch.int32)
+    cu_k = torch.tensor([0] + list(np.cumsum(k_lens)), dtype=torch.int32)
+    q, k, v = seeded_qkv(41, (sum(q_lens), Hq, D), (sum(k_lens), Hkv, D), torch.bfloat16)
+    bm = O.block_mask(Hq, 8192, **pk)
+    ref, ref_lse = O.varlen_attention(q.float(), k.float(), v.float(), cu_k, bm, bs, cu_seqlens_q=cu_q)
+    mod = _module(Hq, 8192, pk, impl="sm100")
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        out, lse = mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda(), return_lse=True)
+    assert_out_close(out, ref)
+    assert_lse_close(lse, ref_lse)
