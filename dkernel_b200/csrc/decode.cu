@@ -2,15 +2,15 @@
 //
 // Grid = (split, kv head x head group, sequence).  A CTA owns up to
 // blocks_per_split attended blocks of one (sequence, kv head): a producer warp
-// streams their K and V tiles (64 tokens x D, 128-byte-swizzled TMA boxes) through
-// a 2-stage shared-memory ring (three CTAs fit per SM, so one CTA's prologue and epilogue
-// are covered by the loads of the other two), and four consumer warps each take 16 tokens of
-// every tile.  The q heads of the kv group are stacked into the 16 rows of an
-// m16n8k16 tensor-core tile, so K/V are read from HBM once per group, and the
-// per-token work is a handful of ldmatrix + mma instructions, which keeps the
-// kernel on the memory roofline.  Each warp keeps its own online-softmax state;
-// warps are merged through shared memory at the end and the CTA writes either
-// the final (O, LSE) (one split) or an fp32 partial that merge_kernel combines.
+// streams their K and V tiles (TMA boxes of kTok tokens x D) through a 64 KB
+// shared-memory ring (three CTAs fit per SM, so one CTA's prologue and epilogue
+// are covered by the loads of the other two).  Every tile pair ("unit") belongs to ONE of the
+// four consumer warps, so four units are worked on at a time and the fixed costs of a unit
+// (barrier, maximum over the tokens, rescaling) are paid once per unit instead of once per warp.
+// The products are transposed, S^T = K Q^T and O^T = V^T P^T, which puts the tokens (and the
+// head dims) on the 16 rows of an m16n8k16 product and the q heads of the kv group on its 8
+// columns: K/V are read from HBM once per group, and a group of four heads wastes half of a
+// product instead of three quarters.
 //
 // Semantics follow the q_len == 1 case of
 // dkernel/ops/sparse_attn_inference.py:503-514: positions are re-based to the
@@ -29,12 +29,12 @@ __device__ __align__(16) int g_wait_status[4] = {0, 0, 0, 0};
 
 namespace {
 
-constexpr int kStages = 2;               // K/V ring depth
+constexpr int kRingBytes = 65536;        // K/V ring
 constexpr int kMinCtas = 3;              // resident CTAs per SM the kernel is built for
-constexpr int kTok = 64;                 // tokens per pipeline stage
 constexpr int kConsumers = 4;            // consumer warps
 constexpr int kDecThreads = 32 * (kConsumers + 1);
-constexpr int kMaxUnits = 64;            // stage-units per CTA
+constexpr int kMaxTokens = 4096;         // tokens per CTA
+constexpr float kDecRescale = 8.0f;      // log2 of how far a maximum may grow before O is rescaled
 
 template <typename T> struct MmaType;
 template <> struct MmaType<__half> {
@@ -79,46 +79,63 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t&
                : "r"(addr));
 }
 
-struct DecodeSmem {
-  // after the 1024-aligned stage ring
-  uint64_t full[2 * kStages];   // the 8-bit K/V ring is twice as deep
-  uint64_t empty[2 * kStages];
-  int n_units;              // stage-units of this CTA
-  int unit_pos[kMaxUnits];  // first position of each stage-unit
-  float wm[kConsumers][16];
-  float wl[kConsumers][16];
-};
-
-// byte offset of 16-byte chunk `chunk` (0 .. D/8-1) of token row `tok` in a tile
-// stored as D/64 sub-tiles of [64 tokens][128 bytes], 128-byte swizzled
-__device__ __forceinline__ uint32_t tile_off(int tok, int chunk) {
-  return (uint32_t)((chunk >> 3) * (kTok * 128) + tok * 128 + (((chunk & 7) ^ (tok & 7)) << 4));
+// transpose of an 8x8 tile of 16-bit elements held in fragment form (two elements per thread)
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
+  return d;
+}
+__device__ __forceinline__ float dec_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // Shared-memory geometry.  16-bit K/V: a stage holds a K and a V tile as the tensor cores read
-// them (D/64 sub-tiles of [64 tokens][128 bytes], 128-byte swizzled).  8-bit (e4m3) K/V: a stage
-// holds the two tiles as stored ([64 tokens][D bytes], half the bytes, so twice the stages keep
-// the same number of bytes in flight); the consumer warps read the stored bytes with plain
+// them (D/64 sub-tiles of [kTok tokens][128 bytes], 128-byte swizzled).  8-bit (e4m3) K/V: a stage
+// holds the two tiles as stored ([kTok tokens][D bytes]; 128-byte rows are swizzled, which keeps
+// the V reads below free of bank conflicts); the consumer warps read the stored bytes with plain
 // 16-byte loads and convert them straight into tensor-core fragments in registers.  e4m3 converts
 // to f16 exactly and in one instruction per pair, so with an 8-bit cache the products run in f16
-// whatever the type of q (q is converted once while it is staged; P lies in [0, 1]).
+// whatever the type of q (q is converted once while it is staged; P lies in [0, 2^kDecRescale]).
 //
 // Fragment trick of the 8-bit path: a product's contraction index may be enumerated in any order,
-// and so may the output columns, as long as both operands (resp. the epilogue) agree.
-//   Q K^T: thread (g, tq) of an m16n8k16 step holds k slots {2tq, 2tq+1, 8+2tq, 9+2tq}.  Over the
+// and so may the output rows, as long as both operands (resp. the epilogue) agree.
+//   K Q^T: thread (g, tq) of an m16n8k16 step holds k slots {2tq, 2tq+1, 8+2tq, 9+2tq}.  Over the
 //          four steps of a 64-dim chunk these are made to stand for dims 16 tq .. 16 tq + 15 of the
 //          chunk (step kk: dims 16 tq + 4 kk + {0,1} and + {2,3}), so a thread's share of a K row
-//          is ONE 16-byte load and each of its four words converts into one step's B fragment.
-//   P V:   output column j of n-tile nt stands for dim (D/8) j + nt, so thread g owns D/8
-//          consecutive dims: its share of a V row is one 16-byte (D = 128) load, and a byte
-//          permute pairs the bytes of two token rows into the B fragment of an n-tile.
+//          is ONE 16-byte load and each of its four words converts into one step's A fragment.
+//   V^T P^T: rows g and g + 8 of m-tile md stand for dims (D/8) g + 2 md and + 1, so thread g owns
+//          D/8 consecutive dims: its share of a V row is one 16-byte (D = 128) load, and a byte
+//          permute pairs the bytes of two token rows into the A fragment of an m-tile.
 template <int D, bool FP8> struct DecGeo {
-  static constexpr int kStages = FP8 ? 2 * bsa::kStages : bsa::kStages;
+  static constexpr int kTok = D == 128 && !FP8 ? 32 : 64;   // tokens per unit
   static constexpr int kTileBytes = kTok * D * (FP8 ? 1 : 2);
   static constexpr int kStageBytes = 2 * kTileBytes;
-  static constexpr int kRing = kStages * kStageBytes;
-  static constexpr size_t kSmem = 1024 + kRing + 16 * D * 2 + sizeof(DecodeSmem);
+  static constexpr int kStages = kRingBytes / kStageBytes;
+  static constexpr int kMaxUnits = kMaxTokens / kTok;       // units per CTA
+  static constexpr bool kSwizzle = !FP8 || D == 128;
+  static_assert(kStages % kConsumers == 0, "a stage belongs to one consumer warp");
+  // byte offset of 16-byte chunk `chunk` of token row `tok` in a tile
+  static __device__ __forceinline__ uint32_t off(int tok, int chunk) {
+    if (FP8) return (uint32_t)(tok * D + ((kSwizzle ? chunk ^ (tok & 7) : chunk) << 4));
+    return (uint32_t)((chunk >> 3) * (kTok * 128) + tok * 128 + (((chunk & 7) ^ (tok & 7)) << 4));
+  }
 };
+
+template <int D, bool FP8, int NT> struct DecodeSmem {
+  // after the 1024-aligned ring
+  alignas(16) uint16_t q[NT * 8][D];           // q heads of the group, zero rows behind them
+  uint64_t full[DecGeo<D, FP8>::kStages];
+  uint64_t empty[DecGeo<D, FP8>::kStages];
+  int n_units;                                 // units of this CTA
+  int unit_pos[DecGeo<D, FP8>::kMaxUnits];     // first position of each unit
+  float wm[kConsumers][NT * 8];
+  float wl[kConsumers][NT * 8];
+};
+template <int D, bool FP8, int NT> constexpr size_t dec_smem() {
+  return 1024 + kRingBytes + sizeof(DecodeSmem<D, FP8, NT>);
+}
 
 // four e4m3 bytes of a word -> two f16x2: (byte 0, byte 1) and (byte 2, byte 3); exact
 __device__ __forceinline__ void cvt_e4m3x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
@@ -132,12 +149,19 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
   return d;
 }
 
-template <typename T, int D, bool FP8>
-__global__ void __launch_bounds__(kDecThreads, kMinCtas)
+// NT: 8-column tiles of q heads (heads_per_cta <= 8 NT).
+//
+// Bound by HBM with a 16-bit cache; with an 8-bit cache by the latency of the consumer warps and the
+// fixed cost of a CTA (row lookup, first tile, merge of the warps: 6 us).  64 sequences of 1024..8192
+// tokens, 32/8 heads, D 128, local 16 + stride 8: 63 us for the 401 MB of a bf16 cache (6.3 TB/s), 48 us
+// for the 203 MB of an e4m3 cache; 71 and 72 us when all four warps shared a unit, 16 tokens each,
+// with the heads on the rows (per unit and warp 2000 cycles of arithmetic latency, four times over).
+template <typename T, int D, bool FP8, int NT>
+__global__ void __launch_bounds__(kDecThreads, FP8 && D == 128 && NT == 2 ? 2 : kMinCtas)   // 2: spills otherwise
 decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 tmV,
               bsa_decode_params p, int nsplit, int* wait_status) {
   using Geo = DecGeo<D, FP8>;
-  constexpr int kStages = Geo::kStages;
+  constexpr int kStages = Geo::kStages, kTok = Geo::kTok;
   constexpr int kTileBytes = Geo::kTileBytes;
   constexpr int kStageBytes = Geo::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -145,8 +169,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
                                              ~uintptr_t(1023));
   uint8_t* ring = smem;
   using MT = typename std::conditional<FP8, __half, T>::type;   // type of the tensor-core products
-  MT* Qs = reinterpret_cast<MT*>(smem + Geo::kRing);  // [16][D]
-  DecodeSmem* sm = reinterpret_cast<DecodeSmem*>(smem + Geo::kRing + 16 * D * 2);
+  auto* sm = reinterpret_cast<DecodeSmem<D, FP8, NT>*>(smem + kRingBytes);
 
   // the merge kernel behind this one may be made resident as soon as every CTA got here
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -181,7 +204,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     (void)BSA_IN_BOUNDS(tok >= 0 && tok < p.sk && kvh >= 0 && kvh < p.hkv && b < p.batch, wait_status, 821);
     uint8_t* kdst = ring + s * kStageBytes;
     uint8_t* vdst = kdst + kTileBytes;
-    if (FP8) {   // one box of [64 tokens][D bytes] per tensor, as stored
+    if (FP8) {   // one box of [kTok tokens][D bytes] per tensor, as stored
       tma_load_tile(kdst, &tmK, &sm->full[s], 0, tok, kvh, b);
       tma_load_tile(vdst, &tmV, &sm->full[s], 0, tok, kvh, b);
     } else {
@@ -224,7 +247,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
             // positions grow with the entry index, so the units past the end form a tail
             const int pos = c * bs + s * kTok;
             const int u = (idx - want0) * subs + s;
-            if (pos < end_pos && u < kMaxUnits) {
+            if (pos < end_pos && u < Geo::kMaxUnits) {
               sm->unit_pos[u] = pos;
               ++valid_units;
             }
@@ -239,14 +262,14 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       sm->n_units = nu;
       for (int s = 0; s < kStages; ++s) {
         mbar_init(&sm->full[s], 1);
-        mbar_init(&sm->empty[s], kConsumers);
+        mbar_init(&sm->empty[s], 1);   // the warp that owns the unit
       }
       mbar_fence_init();
       for (int u = 0; u < nu && u < kStages; ++u) issue_unit(u);
     }
   } else {
-    // q heads of the group -> rows of the 16-row A tile (rows >= GH are zero), 16 bytes a thread
-    for (int i = tid; i < 16 * D / 8; i += kConsumers * 32) {
+    // q heads of the group -> rows of the q tile (rows >= GH are zero), 16 bytes a thread
+    for (int i = tid; i < NT * 8 * D / 8; i += kConsumers * 32) {
       const int r = i / (D / 8), c = i % (D / 8);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < GH) {
@@ -254,20 +277,20 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         if (q_vec) {
           v = *reinterpret_cast<const uint4*>(src);
         } else {
-          T tmp[8];
+          alignas(16) T tmp[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) tmp[e] = src[e];
           v = *reinterpret_cast<const uint4*>(tmp);
         }
         if (!std::is_same<MT, T>::value) {   // bf16 queries against an 8-bit cache: products run in f16
           const T* e = reinterpret_cast<const T*>(&v);
-          __half hq[8];
+          alignas(16) __half hq[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) hq[j] = __float2half_rn(fminf(fmaxf(Elem<T>::to_f(e[j]), -65504.f), 65504.f));
           v = *reinterpret_cast<const uint4*>(hq);
         }
       }
-      reinterpret_cast<uint4*>(Qs)[i] = v;
+      reinterpret_cast<uint4*>(&sm->q[0][0])[i] = v;
     }
   }
   __syncthreads();
@@ -296,9 +319,11 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   }
 
   const int g = lane >> 2, tq = lane & 3;
-  float oacc[D / 8][4];
+  float oacc[D / 16][NT][4];   // O^T: rows = dims, columns = heads
 #pragma unroll
-  for (int i = 0; i < D / 8; ++i) oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f;
+  for (int i = 0; i < D / 16; ++i)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) oacc[i][nt][0] = oacc[i][nt][1] = oacc[i][nt][2] = oacc[i][nt][3] = 0.f;
 
   if (warp == kConsumers) {
     // ------------------------------------------------------------ producer
@@ -312,214 +337,253 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     }
   } else {
     // ------------------------------------------------------------ consumers
-    uint32_t qa[D / 16][4];
+    uint32_t qb[D / 16][NT][2];   // Q^T as the B operand: column n = g is head 8 nt + g
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      const uint32_t* q32 = reinterpret_cast<const uint32_t*>(Qs);
-      // k slots (2tq, 2tq+1) and (8+2tq, 9+2tq) of step kk: the dims of the same numbers, or
-      // (8-bit K/V) dims 16 tq + 4 (kk % 4) + {0,1} / {2,3} of 64-dim chunk kk / 4
-      const int d0 = FP8 ? (kk >> 2) * 64 + tq * 16 + (kk & 3) * 4 : kk * 16 + tq * 2;
-      const int d1 = FP8 ? d0 + 2 : d0 + 8;
-      qa[kk][0] = q32[(g * D + d0) >> 1];
-      qa[kk][1] = q32[((g + 8) * D + d0) >> 1];
-      qa[kk][2] = q32[(g * D + d1) >> 1];
-      qa[kk][3] = q32[((g + 8) * D + d1) >> 1];
-    }
-    float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
+    for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const uint32_t* q32 = reinterpret_cast<const uint32_t*>(sm->q[nt * 8 + g]);
+        // k slots (2tq, 2tq+1) and (8+2tq, 9+2tq) of step kk: the dims of the same numbers, or
+        // (8-bit K/V) dims 16 tq + 4 (kk % 4) + {0,1} / {2,3} of 64-dim chunk kk / 4
+        const int d0 = FP8 ? (kk >> 2) * 64 + tq * 16 + (kk & 3) * 4 : kk * 16 + tq * 2;
+        const int d1 = FP8 ? d0 + 2 : d0 + 8;
+        qb[kk][nt][0] = q32[d0 >> 1];
+        qb[kk][nt][1] = q32[d1 >> 1];
+      }
+    // per head 8 nt + 2 tq + e: reference maximum (log2 domain), this thread's share of the sum
+    float m[NT][2], l[NT][2];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) { m[nt][0] = m[nt][1] = -INFINITY; l[nt][0] = l[nt][1] = 0.f; }
     // e4m3 K carries a per-tensor scale: it folds into the logit scale (V's goes on the output)
     const float scale2 = p.sm_scale * kLog2e * (FP8 ? p.k_scale : 1.f);
     const uint32_t ring_u32 = smem_u32(ring);
-    bool alive = true;
 
-    for (int u = 0; u < n_units && alive; ++u) {
+    for (int u = warp; u < n_units; u += kConsumers) {
       const int s = u % kStages;
       const uint32_t ph = (u / kStages) & 1;
-      alive = mbar_wait(&sm->full[s], ph, wait_status, 102);
-      if (!alive) break;
-      const int pos_u = sm->unit_pos[u];
+      if (!mbar_wait(&sm->full[s], ph, wait_status, 102)) break;
       const uint32_t kbase = ring_u32 + s * kStageBytes;
       const uint32_t vbase = kbase + kTileBytes;
-      const int valid = end_pos - pos_u;  // tokens of this unit that exist (may exceed 64)
       const uint8_t* k8 = ring + s * kStageBytes;    // the tiles as generic pointers (8-bit path)
       const uint8_t* v8 = k8 + kTileBytes;
-      if (FP8) {
-        // nothing to prepare: rows past the end of the sequence are zeroed when V is read
-      } else if (valid < kTok) {
-        // rows past the end of the sequence may hold anything: clear them in V so
-        // that 0 * garbage cannot produce NaN
+      const int valid = end_pos - sm->unit_pos[u];   // tokens of this unit that exist (may exceed kTok)
+      if (!FP8 && valid < kTok) {
+        // rows past the end of the sequence may hold anything: clear them in V so that 0 * garbage
+        // cannot produce NaN (the 8-bit path replaces them as it reads V)
         uint8_t* vgen = ring + s * kStageBytes + kTileBytes;
-        for (int t = warp * 16; t < warp * 16 + 16; ++t) {
-          if (t >= valid) {
+        for (int t = valid; t < kTok; ++t)
 #pragma unroll
-            for (int c = 0; c < D / 64; ++c)
-              reinterpret_cast<uint32_t*>(vgen + c * (kTok * 128) + t * 128)[lane] = 0u;
-          }
-        }
+          for (int c = 0; c < D / 64; ++c)
+            reinterpret_cast<uint32_t*>(vgen + c * (kTok * 128) + t * 128)[lane] = 0u;
         fence_proxy_async();  // order these writes before the next TMA into the stage
         __syncwarp();
       }
-      // S = Q K^T for this warp's 16 tokens
-      float sacc[2][4];
+      // S^T = K Q^T
+      float sacc[kTok / 16][NT][4];
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        sacc[nt][0] = sacc[nt][1] = sacc[nt][2] = sacc[nt][3] = 0.f;
+      for (int mt = 0; mt < kTok / 16; ++mt) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) sacc[mt][nt][0] = sacc[mt][nt][1] = sacc[mt][nt][2] = sacc[mt][nt][3] = 0.f;
         if (FP8) {
-          const int tok = warp * 16 + nt * 8 + g;      // B fragment column n = g
 #pragma unroll
           for (int c = 0; c < D / 64; ++c) {
-            const uint4 kb = *reinterpret_cast<const uint4*>(k8 + tok * D + c * 64 + tq * 16);
-            const uint32_t w[4] = {kb.x, kb.y, kb.z, kb.w};
+            const uint4 lo = *reinterpret_cast<const uint4*>(k8 + Geo::off(mt * 16 + g, c * 4 + tq));
+            const uint4 hi = *reinterpret_cast<const uint4*>(k8 + Geo::off(mt * 16 + g + 8, c * 4 + tq));
+            const uint32_t wl[4] = {lo.x, lo.y, lo.z, lo.w}, wh[4] = {hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-              uint32_t b0, b1;
-              cvt_e4m3x4(w[kk], b0, b1);
-              MmaType<MT>::mma(sacc[nt], qa[c * 4 + kk], b0, b1);
+              uint32_t a[4];
+              cvt_e4m3x4(wl[kk], a[0], a[2]);
+              cvt_e4m3x4(wh[kk], a[1], a[3]);
+#pragma unroll
+              for (int nt = 0; nt < NT; ++nt)
+                MmaType<MT>::mma(sacc[mt][nt], a, qb[c * 4 + kk][nt][0], qb[c * 4 + kk][nt][1]);
             }
           }
         } else {
-          const int tok = warp * 16 + nt * 8 + (lane & 7);
 #pragma unroll
-          for (int kk = 0; kk < D / 32; ++kk) {
-            uint32_t r0, r1, r2, r3;
-            ldsm_x4(kbase + tile_off(tok, kk * 4 + (lane >> 3)), r0, r1, r2, r3);
-            MmaType<MT>::mma(sacc[nt], qa[2 * kk], r0, r1);
-            MmaType<MT>::mma(sacc[nt], qa[2 * kk + 1], r2, r3);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            uint32_t a[4];
+            ldsm_x4(kbase + Geo::off(mt * 16 + (lane & 15), kk * 2 + (lane >> 4)), a[0], a[1], a[2], a[3]);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) MmaType<MT>::mma(sacc[mt][nt], a, qb[kk][nt][0], qb[kk][nt][1]);
           }
         }
       }
-      // mask + online softmax (rows g and g+8)
-      float mx_lo = -INFINITY, mx_hi = -INFINITY;
+      // mask; per head: maximum over the unit's tokens, reference maximum, sum
+      float alpha[NT][2];
+      bool need = false;
+      if (valid < kTok) {
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
+        for (int mt = 0; mt < kTok / 16; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (mt * 16 + g + (e >> 1) * 8 >= valid) sacc[mt][nt][e] = -INFINITY;
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const int t = warp * 16 + nt * 8 + tq * 2 + e;
-          const bool ok = t < valid;
-          sacc[nt][e] = ok ? sacc[nt][e] * scale2 : -INFINITY;
-          sacc[nt][2 + e] = ok ? sacc[nt][2 + e] * scale2 : -INFINITY;
-          mx_lo = fmaxf(mx_lo, sacc[nt][e]);
-          mx_hi = fmaxf(mx_hi, sacc[nt][2 + e]);
-        }
-      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
-      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-      const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
-      const float ms_lo = mn_lo == -INFINITY ? 0.f : mn_lo;
-      const float ms_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
-      const float a_lo = exp2f(m_lo - ms_lo), a_hi = exp2f(m_hi - ms_hi);
-      m_lo = mn_lo;
-      m_hi = mn_hi;
-      uint32_t pa[4];
-      {
-        const float p00 = exp2f(sacc[0][0] - ms_lo), p01 = exp2f(sacc[0][1] - ms_lo);
-        const float p02 = exp2f(sacc[0][2] - ms_hi), p03 = exp2f(sacc[0][3] - ms_hi);
-        const float p10 = exp2f(sacc[1][0] - ms_lo), p11 = exp2f(sacc[1][1] - ms_lo);
-        const float p12 = exp2f(sacc[1][2] - ms_hi), p13 = exp2f(sacc[1][3] - ms_hi);
-        l_lo = l_lo * a_lo + (p00 + p01 + p10 + p11);
-        l_hi = l_hi * a_hi + (p02 + p03 + p12 + p13);
-        pa[0] = MmaType<MT>::pack(p00, p01);
-        pa[1] = MmaType<MT>::pack(p02, p03);
-        pa[2] = MmaType<MT>::pack(p10, p11);
-        pa[3] = MmaType<MT>::pack(p12, p13);
-      }
+          float mx = -INFINITY;
 #pragma unroll
-      for (int i = 0; i < D / 8; ++i) {
-        oacc[i][0] *= a_lo; oacc[i][1] *= a_lo;
-        oacc[i][2] *= a_hi; oacc[i][3] *= a_hi;
-      }
-      // O += P V over this warp's 16 tokens
-      if (FP8) {
-        // k slots (2tq, 2tq+1, 8+2tq, 9+2tq) are this warp's token rows of the same numbers; the
-        // thread's D/8 consecutive dims of each row arrive in one load (zero past the sequence end)
-        constexpr int kNT = D / 8;                       // n-tiles = dims per thread
-        uint32_t rows[4][kNT / 4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int tok = warp * 16 + (i >> 1) * 8 + tq * 2 + (i & 1);
-          const uint8_t* src = v8 + tok * D + g * kNT;
-          if (kNT == 16) {
-            const uint4 r = tok < valid ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);
-            rows[i][0] = r.x; rows[i][1] = r.y; rows[i][kNT / 4 - 2] = r.z; rows[i][kNT / 4 - 1] = r.w;
-          } else {
-            const uint2 r = tok < valid ? *reinterpret_cast<const uint2*>(src) : make_uint2(0u, 0u);
-            rows[i][0] = r.x; rows[i][kNT / 4 - 1] = r.y;
+          for (int mt = 0; mt < kTok / 16; ++mt) mx = fmaxf(mx, fmaxf(sacc[mt][nt][e], sacc[mt][nt][2 + e]));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+          mx *= scale2;
+          alpha[nt][e] = 1.f;
+          if (m[nt][e] == -INFINITY) {
+            m[nt][e] = mx;         // nothing summed so far
+          } else if (mx > m[nt][e] + kDecRescale) {
+            alpha[nt][e] = dec_ex2(m[nt][e] - mx);
+            m[nt][e] = mx;
+            need = true;
           }
         }
+      if (__any_sync(0xffffffffu, need)) {
 #pragma unroll
-        for (int nt2 = 0; nt2 < kNT / 2; ++nt2) {         // two n-tiles (dims 2 nt2, 2 nt2 + 1 of the thread) per permute
-          const int wi = nt2 >> 1;
-          const uint32_t sel = (nt2 & 1) ? 0x7362u : 0x5140u;   // {a.b, b.b, a.b+1, b.b+1}, b = 0 or 2
-          uint32_t b0a, b0b, b1a, b1b;
-          cvt_e4m3x4(byte_perm(rows[0][wi], rows[1][wi], sel), b0a, b0b);   // tokens 2tq, 2tq+1
-          cvt_e4m3x4(byte_perm(rows[2][wi], rows[3][wi], sel), b1a, b1b);   // tokens 8+2tq, 9+2tq
-          MmaType<MT>::mma(oacc[2 * nt2], pa, b0a, b1a);
-          MmaType<MT>::mma(oacc[2 * nt2 + 1], pa, b0b, b1b);
+        for (int nt = 0; nt < NT; ++nt) {
+          l[nt][0] *= alpha[nt][0];
+          l[nt][1] *= alpha[nt][1];
+#pragma unroll
+          for (int i = 0; i < D / 16; ++i) {
+            oacc[i][nt][0] *= alpha[nt][0]; oacc[i][nt][1] *= alpha[nt][1];
+            oacc[i][nt][2] *= alpha[nt][0]; oacc[i][nt][3] *= alpha[nt][1];
+          }
         }
-      } else {
+      }
+      // P^T as the B operand: the 8x8 tiles of S^T's accumulator layout, transposed
+      uint32_t pb[kTok / 16][NT][2];
 #pragma unroll
-        for (int dn = 0; dn < D / 16; ++dn) {
-          const int mi = lane >> 3;
-          const int tok = warp * 16 + (mi & 1) * 8 + (lane & 7);
-          uint32_t r0, r1, r2, r3;
-          ldsm_x4_t(vbase + tile_off(tok, dn * 2 + (mi >> 1)), r0, r1, r2, r3);
-          MmaType<MT>::mma(oacc[2 * dn], pa, r0, r1);
-          MmaType<MT>::mma(oacc[2 * dn + 1], pa, r2, r3);
+      for (int nt = 0; nt < NT; ++nt) {
+        const float n0 = m[nt][0] == -INFINITY ? 0.f : -m[nt][0], n1 = m[nt][1] == -INFINITY ? 0.f : -m[nt][1];
+#pragma unroll
+        for (int mt = 0; mt < kTok / 16; ++mt) {
+          const float p0 = dec_ex2(fmaf(sacc[mt][nt][0], scale2, n0)), p1 = dec_ex2(fmaf(sacc[mt][nt][1], scale2, n1));
+          const float p2 = dec_ex2(fmaf(sacc[mt][nt][2], scale2, n0)), p3 = dec_ex2(fmaf(sacc[mt][nt][3], scale2, n1));
+          l[nt][0] += p0 + p2;
+          l[nt][1] += p1 + p3;
+          pb[mt][nt][0] = transpose8x8(MmaType<MT>::pack(p0, p1));
+          pb[mt][nt][1] = transpose8x8(MmaType<MT>::pack(p2, p3));
+        }
+      }
+      // O^T += V^T P^T
+#pragma unroll
+      for (int mt = 0; mt < kTok / 16; ++mt) {
+        if (FP8) {
+          // k slots (2tq, 2tq+1, 8+2tq, 9+2tq) are the token rows of the same numbers; the thread's
+          // D/8 consecutive dims of each row arrive in one load (zero past the sequence end)
+          constexpr int kDims = D / 8;
+          uint32_t rows[4][kDims / 4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int tok = mt * 16 + (i >> 1) * 8 + tq * 2 + (i & 1);
+            if (kDims == 16) {
+              const uint4 r = tok < valid ? *reinterpret_cast<const uint4*>(v8 + Geo::off(tok, g))
+                                          : make_uint4(0u, 0u, 0u, 0u);
+              rows[i][0] = r.x; rows[i][1] = r.y; rows[i][kDims / 4 - 2] = r.z; rows[i][kDims / 4 - 1] = r.w;
+            } else {
+              const uint2 r = tok < valid ? *reinterpret_cast<const uint2*>(v8 + tok * D + g * kDims)
+                                          : make_uint2(0u, 0u);
+              rows[i][0] = r.x; rows[i][kDims / 4 - 1] = r.y;
+            }
+          }
+#pragma unroll
+          for (int md = 0; md < D / 16; ++md) {
+            const int wi = md >> 1;
+            const uint32_t sel = (md & 1) ? 0x7362u : 0x5140u;   // {a.b, b.b, a.b+1, b.b+1}, b = 0 or 2
+            uint32_t a[4];
+            cvt_e4m3x4(byte_perm(rows[0][wi], rows[1][wi], sel), a[0], a[1]);   // tokens 2tq, 2tq+1
+            cvt_e4m3x4(byte_perm(rows[2][wi], rows[3][wi], sel), a[2], a[3]);   // tokens 8+2tq, 9+2tq
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) MmaType<MT>::mma(oacc[md][nt], a, pb[mt][nt][0], pb[mt][nt][1]);
+          }
+        } else {
+#pragma unroll
+          for (int md = 0; md < D / 16; ++md) {
+            const int j = lane >> 3;
+            uint32_t a[4];
+            ldsm_x4_t(vbase + Geo::off(mt * 16 + (j >> 1) * 8 + (lane & 7), md * 2 + (j & 1)), a[0], a[1], a[2], a[3]);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) MmaType<MT>::mma(oacc[md][nt], a, pb[mt][nt][0], pb[mt][nt][1]);
+          }
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm->empty[s]);
     }
-    // quad-reduce the row sums
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-    if (tq == 0) {
-      sm->wm[warp][g] = m_lo; sm->wm[warp][g + 8] = m_hi;
-      sm->wl[warp][g] = l_lo; sm->wl[warp][g + 8] = l_hi;
-    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) l[nt][e] += __shfl_xor_sync(0xffffffffu, l[nt][e], o);
+        if (g == 0) {
+          sm->wm[warp][nt * 8 + 2 * tq + e] = m[nt][e];
+          sm->wl[warp][nt * 8 + 2 * tq + e] = l[nt][e];
+        }
+      }
   }
   __syncthreads();  // every tile has been consumed: the ring is free
+  // partial outputs, [warp][head][D]; four floats of padding per row spread the writes over the banks
+  constexpr int kRow = D + 4;
+  float* Om = reinterpret_cast<float*>(ring);
+  static_assert(kConsumers * NT * 8 * kRow * 4 <= kRingBytes, "partial outputs must fit the ring");
   if (warp < kConsumers) {
-    float* Omw = reinterpret_cast<float*>(ring);  // [kConsumers][16][D]
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      // column j = 2tq (+1) of n-tile i is dim 8 i + j, or (8-bit K/V) dim (D/8) j + i
-      const int d0 = FP8 ? (D / 8) * (tq * 2) + i : i * 8 + tq * 2;
-      const int d1 = FP8 ? d0 + D / 8 : d0 + 1;
-      float* lo = Omw + ((warp * 16 + g) * D);
-      float* hi = Omw + ((warp * 16 + g + 8) * D);
-      lo[d0] = oacc[i][0]; lo[d1] = oacc[i][1];
-      hi[d0] = oacc[i][2]; hi[d1] = oacc[i][3];
+    for (int nt = 0; nt < NT; ++nt) {
+      float* h_lo = Om + (warp * NT * 8 + nt * 8 + 2 * tq) * kRow;   // heads 2tq and 2tq + 1
+      float* h_hi = h_lo + kRow;
+#pragma unroll
+      for (int md = 0; md < D / 16; ++md) {
+        // rows g and g + 8 of m-tile md: the dims of the same numbers, or (8-bit K/V) two neighbours
+        const int d0 = FP8 ? (D / 8) * g + 2 * md : md * 16 + g;
+        const int d1 = FP8 ? d0 + 1 : d0 + 8;
+        h_lo[d0] = oacc[md][nt][0]; h_hi[d0] = oacc[md][nt][1];
+        h_lo[d1] = oacc[md][nt][2]; h_hi[d1] = oacc[md][nt][3];
+      }
     }
   }
   __syncthreads();  // partial outputs are in shared memory
 
-  const float* Om = reinterpret_cast<const float*>(ring);
-  for (int i = tid; i < GH * D; i += kDecThreads) {
-    const int r = i / D, d = i % D;
+  const bool o_vec = reinterpret_cast<uintptr_t>(p.o) % 8 == 0 && p.o_sb % 4 == 0 && p.o_sh % 4 == 0;
+  const bool ws_vec = reinterpret_cast<uintptr_t>(p.ws) % 16 == 0;
+  for (int i = tid; i < GH * (D / 4); i += kDecThreads) {
+    const int r = i / (D / 4), d = i % (D / 4) * 4;
     float mf = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kConsumers; ++w) mf = fmaxf(mf, sm->wm[w][r]);
     const float msafe = mf == -INFINITY ? 0.f : mf;
-    float acc = 0.f, l = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
 #pragma unroll
     for (int w = 0; w < kConsumers; ++w) {
       const float sc = exp2f(sm->wm[w][r] - msafe);
-      acc += Om[(w * 16 + r) * D + d] * sc;
+      const float4 v = *reinterpret_cast<const float4*>(Om + (w * NT * 8 + r) * kRow + d);
+      acc.x += v.x * sc; acc.y += v.y * sc; acc.z += v.z * sc; acc.w += v.w * sc;
       l += sm->wl[w][r] * sc;
     }
     const float inv = (l > 0.f ? 1.f / l : 0.f) * (FP8 ? p.v_scale : 1.f);   // e4m3 V: per-tensor scale
     const float lse = l > 0.f ? (mf + log2f(l)) * kLn2 : -INFINITY;
+    acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
     const int h = h0 + r;
     if (final_out) {
-      reinterpret_cast<T*>(p.o)[(int64_t)b * p.o_sb + (int64_t)h * p.o_sh + d] =
-          Elem<T>::from_f(acc * inv);
+      T* dst = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + d;
+      if (o_vec) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(MmaType<T>::pack(acc.x, acc.y), MmaType<T>::pack(acc.z, acc.w));
+      } else {
+        dst[0] = Elem<T>::from_f(acc.x); dst[1] = Elem<T>::from_f(acc.y);
+        dst[2] = Elem<T>::from_f(acc.z); dst[3] = Elem<T>::from_f(acc.w);
+      }
       if (d == 0 && p.lse) p.lse[(int64_t)b * p.lse_sb + (int64_t)h * p.lse_sh] = lse;
     } else {
-      if (BSA_IN_BOUNDS(h < p.hq && sp < nsplit && d < D, wait_status, 822))
-        p.ws[(((int64_t)b * p.hq + h) * nsplit + sp) * D + d] = acc * inv;
+      if (BSA_IN_BOUNDS(h < p.hq && sp < nsplit && d < D, wait_status, 822)) {
+        float* dst = p.ws + (((int64_t)b * p.hq + h) * nsplit + sp) * D + d;
+        if (ws_vec) *reinterpret_cast<float4*>(dst) = acc;
+        else { dst[0] = acc.x; dst[1] = acc.y; dst[2] = acc.z; dst[3] = acc.w; }
+      }
       if (d == 0)
         p.ws[(int64_t)p.batch * p.hq * nsplit * D + ((int64_t)b * p.hq + h) * nsplit + sp] = lse;
     }
@@ -618,21 +682,22 @@ int decode_nsplit(const bsa_decode_params* p) {
   return n < 1 ? 1 : n;
 }
 
-template <typename T, int D, bool FP8>
+template <typename T, int D, bool FP8, int NT>
 int launch_decode(const bsa_decode_params* p, cudaStream_t s) {
   Tmap4 tmK, tmV;
   const bool bf16 = p->dtype == BSA_BF16;
   const int eb = FP8 ? 1 : 2;
-  const uint32_t box_d = FP8 ? D : 64;    // 8-bit tiles are copied as stored, 16-bit ones 128-byte swizzled
+  using Geo = DecGeo<D, FP8>;
+  const uint32_t box_d = FP8 ? D : 64;    // 8-bit tiles are copied in one box, 16-bit ones in 128-byte wide boxes
   int rc = make_tmap_4d(&tmK, p->k, eb, D, p->sk, p->hkv, p->batch, p->k_ss * eb, p->k_sh * eb,
-                        p->k_sb * eb, box_d, kTok, !FP8, bf16);
+                        p->k_sb * eb, box_d, Geo::kTok, Geo::kSwizzle, bf16);
   if (rc) return rc;
   rc = make_tmap_4d(&tmV, p->v, eb, D, p->sk, p->hkv, p->batch, p->v_ss * eb, p->v_sh * eb,
-                    p->v_sb * eb, box_d, kTok, !FP8, bf16);
+                    p->v_sb * eb, box_d, Geo::kTok, Geo::kSwizzle, bf16);
   if (rc) return rc;
   const int nsplit = decode_nsplit(p);
-  const size_t smem = DecGeo<D, FP8>::kSmem;
-  auto kern = decode_kernel<T, D, FP8>;
+  const size_t smem = dec_smem<D, FP8, NT>();
+  auto kern = decode_kernel<T, D, FP8, NT>;
   BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int G = p->hq / p->hkv;
   dim3 grid(nsplit, p->hkv * (G / p->heads_per_cta), p->batch);
@@ -663,6 +728,16 @@ int launch_decode(const bsa_decode_params* p, cudaStream_t s) {
     return BSA_E_UNSUPPORTED;
   }
   return BSA_OK;
+}
+
+template <typename T>
+int launch_decode_t(const bsa_decode_params* p, bool fp8, cudaStream_t s) {
+  if (p->heads_per_cta > 8) {
+    if (fp8) return p->d == 128 ? launch_decode<T, 128, true, 2>(p, s) : launch_decode<T, 64, true, 2>(p, s);
+    return p->d == 128 ? launch_decode<T, 128, false, 2>(p, s) : launch_decode<T, 64, false, 2>(p, s);
+  }
+  if (fp8) return p->d == 128 ? launch_decode<T, 128, true, 1>(p, s) : launch_decode<T, 64, true, 1>(p, s);
+  return p->d == 128 ? launch_decode<T, 128, false, 1>(p, s) : launch_decode<T, 64, false, 1>(p, s);
 }
 
 }  // namespace
@@ -696,21 +771,14 @@ int decode_run(const bsa_decode_params* p, cudaStream_t s) {
     return BSA_E_UNSUPPORTED;
   }
   const int bps = decode_blocks_per_split(p);
-  if (bps * (p->block_size / kTok) > kMaxUnits) {
-    set_error("bsa_decode: blocks_per_split=%d too large (limit %d tiles of 64 tokens per CTA)", bps,
-              kMaxUnits);
+  if (bps * p->block_size > kMaxTokens) {
+    set_error("bsa_decode: blocks_per_split=%d too large (limit %d tokens per CTA)", bps, kMaxTokens);
     return BSA_E_TOOBIG;
   }
   const int nsplit = decode_nsplit(p);
   BSA_CHECK_ARG((nsplit == 1 && p->o) || p->ws, "bsa_decode: workspace required for %d splits", nsplit);
-  if (fp8) {
-    if (p->dtype == BSA_BF16)
-      return p->d == 128 ? launch_decode<__nv_bfloat16, 128, true>(p, s) : launch_decode<__nv_bfloat16, 64, true>(p, s);
-    return p->d == 128 ? launch_decode<__half, 128, true>(p, s) : launch_decode<__half, 64, true>(p, s);
-  }
-  if (p->dtype == BSA_BF16)
-    return p->d == 128 ? launch_decode<__nv_bfloat16, 128, false>(p, s) : launch_decode<__nv_bfloat16, 64, false>(p, s);
-  return p->d == 128 ? launch_decode<__half, 128, false>(p, s) : launch_decode<__half, 64, false>(p, s);
+  if (p->dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(p, fp8, s);
+  return launch_decode_t<__half>(p, fp8, s);
 }
 
 int merge_partials(const void* o_parts, const float* lse_parts, int P, int64_t rows, int d,

@@ -386,3 +386,34 @@ def test_packed_batch_with_more_than_64k_keys_runs_on_tensor_cores(n_seq, k_len)
         out, lse = mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda(), return_lse=True)
     assert_out_close(out, ref)
     assert_lse_close(lse, ref_lse)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,D,bs,dtype,q_gain", [
+    (4, 4, 128, 64, torch.bfloat16, 1.0),     # one head per group
+    (6, 2, 64, 64, torch.float16, 8.0),       # logits that move the reference maximum
+    (8, 1, 128, 128, torch.bfloat16, 8.0),    # a full 8-column tile
+    (12, 1, 128, 64, torch.float16, 1.0),     # two column tiles, the second one half empty
+    (32, 2, 64, 128, torch.bfloat16, 1.0),    # two full column tiles
+])
+def test_decode_group_sizes_and_unit_edges(fp8, Hq, Hkv, D, bs, dtype, q_gain):
+    """Lengths around the edges of the decode kernel's 32- and 64-token units and of the pattern's blocks,
+    for every number of heads per group that changes how its products are tiled.  The oracle gets the
+    stored (rounded) K/V, so the bounds are those of the 16-bit products: the helpers' defaults."""
+    lens = [1, 31, 32, 33, 63, 64, 65, 127, 129, 257, 500]
+    B, S = len(lens), 512
+    pk = dict(block_size=bs, local_blocks=2, vert_stride=3, num_kv_heads=Hkv)
+    q, k, v = seeded_qkv(61, (B, 1, Hq, D), (B, S, Hkv, D), dtype)
+    q = q * q_gain
+    scales, kw = (0.02, 0.015), {}
+    if fp8:
+        k, v = (k.float() / scales[0]).to(torch.float8_e4m3fn), (v.float() / scales[1]).to(torch.float8_e4m3fn)
+        kw["kv_scales"] = scales
+    kf, vf = (k.float() * scales[0], v.float() * scales[1]) if fp8 else (k.float(), v.float())
+    left = torch.tensor([S - n for n in lens], dtype=torch.int32)
+    ref, ref_lse = O.decode_attention(q.float(), kf, vf, O.block_mask(Hq, S, **pk), bs, left_paddings=left)
+    mod = _module(Hq, S, pk, seq_dim=1)
+    with torch.no_grad():
+        out, lse = mod(q.cuda(), k.cuda(), v.cuda(), left_paddings=left.cuda(), return_lse=True, **kw)
+    assert_out_close(out, ref)
+    assert_lse_close(lse, ref_lse)
