@@ -15,7 +15,7 @@ LIB_PATH = os.environ.get("BSA_B200_LIB") or os.path.join(_HERE, "libbsa_b200.so
 
 BSA_F16, BSA_BF16, BSA_F32, BSA_F8E4M3 = 0, 1, 2, 3
 IMPL_AUTO, IMPL_GENERIC, IMPL_SM100 = 0, 1, 2
-ROWS_BY_TILE, ROWS_BY_POSITION = 0, 1
+ROWS_BY_TILE, ROWS_BY_POSITION, ROWS_BY_POSITION_ZERO_PADS = 0, 1, 2
 
 _i32, _i64, _f32, _vp = C.c_int32, C.c_int64, C.c_float, C.c_void_p
 

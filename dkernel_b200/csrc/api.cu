@@ -21,8 +21,11 @@ int validate_fwd(const bsa_fwd_params* p, const char* who) {
                 "%s: block_size must be a power of two in [16,128], got %d", who, bs);
   BSA_CHECK_ARG(p->dtype == BSA_F16 || p->dtype == BSA_BF16 || p->dtype == BSA_F32,
                 "%s: unknown dtype %d", who, p->dtype);
-  BSA_CHECK_ARG(p->row_mode == BSA_ROWS_BY_TILE || p->row_mode == BSA_ROWS_BY_POSITION,
+  BSA_CHECK_ARG(p->row_mode == BSA_ROWS_BY_TILE || p->row_mode == BSA_ROWS_BY_POSITION ||
+                    p->row_mode == BSA_ROWS_BY_POSITION_ZERO_PADS,
                 "%s: unknown row_mode %d", who, p->row_mode);
+  BSA_CHECK_ARG(p->row_mode != BSA_ROWS_BY_POSITION_ZERO_PADS || (p->q_start && p->q_end && p->total_q == 0),
+                "%s: BSA_ROWS_BY_POSITION_ZERO_PADS is for padded batches (q_start, q_end, total_q = 0)", who);
   BSA_CHECK_ARG((p->q_start == nullptr) == (p->q_end == nullptr) &&
                     (p->k_start == nullptr) == (p->k_end == nullptr),
                 "%s: start/end arrays must be given in pairs", who);
@@ -72,6 +75,10 @@ int bsa_fwd(const bsa_fwd_params* p, void* stream) {
       set_error("bsa_fwd: the tcgen05 kernel does not serve this call: %s", why ? why : "?");
       return BSA_E_UNSUPPORTED;
     }
+  }
+  if (p->row_mode == BSA_ROWS_BY_POSITION_ZERO_PADS) {
+    set_error("bsa_fwd: BSA_ROWS_BY_POSITION_ZERO_PADS is only served by the tcgen05 kernel");
+    return BSA_E_UNSUPPORTED;
   }
   if (p->fine_block != 0) {
     set_error("bsa_fwd: a coarsened fine-block layout (fine_block = %d) is only read by the tcgen05 kernel; "

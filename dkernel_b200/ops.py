@@ -521,11 +521,18 @@ def _padded(q, k, v, sm_scale, plan, left_paddings, seqlens, seq_dim, max_seqlen
     else:
         q_starts, q_ends = k_starts, k_ends
     q, k, v = _tma_friendly(q), _tma_friendly(k), _tma_friendly(v)
-    o = out if out is not None else torch.zeros(q.shape, dtype=q.dtype, device=dev)
-    lse = torch.full((batches, q.size(hdim), q_len), float("-inf"), dtype=torch.float32, device=dev) \
-        if return_lse else None
-    p = _fwd_params(q, k, v, o, lse, seq_dim, plan, sm_scale, causal, _lib.ROWS_BY_POSITION,
+    o = out if out is not None else torch.empty(q.shape, dtype=q.dtype, device=dev)
+    lse = torch.empty((batches, q.size(hdim), q_len), dtype=torch.float32, device=dev) if return_lse else None
+    # pad rows: the tensor-core kernel writes them; a caller's own output keeps what it holds there
+    p = _fwd_params(q, k, v, o, lse, seq_dim, plan, sm_scale, causal,
+                    _lib.ROWS_BY_POSITION_ZERO_PADS if out is None else _lib.ROWS_BY_POSITION,
                     q_starts, q_ends, k_starts, k_ends, impl=impl)
+    if out is not None or _lib.lib().bsa_fwd_uses_sm100(C.byref(p)) != 1:
+        p.row_mode = _lib.ROWS_BY_POSITION
+        if out is None:
+            o.zero_()
+        if lse is not None:
+            lse.fill_(float("-inf"))
     _launch_fwd(p, q)
     return o, lse
 

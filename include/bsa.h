@@ -47,9 +47,13 @@ enum { BSA_IMPL_AUTO = 0, BSA_IMPL_GENERIC = 1, BSA_IMPL_SM100 = 2 };
 enum {
   BSA_ROWS_BY_TILE = 0,    /* row = q tile index (training path,
                               dkernel/ops/sparse_attn_fwd.py:289-291)           */
-  BSA_ROWS_BY_POSITION = 1 /* row = (past_len + tile start) / block, positions
+  BSA_ROWS_BY_POSITION = 1, /* row = (past_len + tile start) / block, positions
                               re-based per sequence (inference path,
                               dkernel/ops/sparse_attn_inference.py:503-514)     */
+  /* As BSA_ROWS_BY_POSITION, for a padded batch (q_start and q_end given, total_q = 0) on the
+   * tcgen05 kernel: the storage rows in front of q_start and behind q_end are written too (zero
+   * rows, LSE = -inf), as dkernel/ops/sparse_attn_inference.py:67 returns them.             */
+  BSA_ROWS_BY_POSITION_ZERO_PADS = 2
 };
 
 int bsa_abi_version(void);

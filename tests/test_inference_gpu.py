@@ -417,3 +417,39 @@ def test_decode_group_sizes_and_unit_edges(fp8, Hq, Hkv, D, bs, dtype, q_gain):
         out, lse = mod(q.cuda(), k.cuda(), v.cuda(), left_paddings=left.cuda(), return_lse=True, **kw)
     assert_out_close(out, ref)
     assert_lse_close(lse, ref_lse)
+
+
+@pytest.mark.parametrize("Hq,Hkv,S,D,bs,seq_dim,lens,right", [
+    (4, 2, 300, 128, 64, 1, [300, 1, 64, 65, 130], False),      # two heads per tile
+    (2, 2, 320, 40, 64, 2, [1, 127, 128, 129, 319], True),      # two row blocks per tile, five pieces a row
+    (4, 4, 257, 64, 32, 1, [63, 256, 191, 2], False),           # fine blocks
+    (2, 1, 130, 256, 64, 2, [5, 130], True),
+])
+def test_pad_rows_of_a_padded_batch_are_written(Hq, Hkv, S, D, bs, seq_dim, lens, right):
+    """The output comes from uninitialised memory: every pad row must be written (zeros, LSE -inf), whatever
+    the memory held; an output that the caller brings keeps its pad rows."""
+    pk = dict(block_size=bs, local_blocks=2, vert_stride=3)
+    B = len(lens)
+    shape = (lambda h: (B, h, S, D)) if seq_dim == 2 else (lambda h: (B, S, h, D))
+    q, k, v = seeded_qkv(71, shape(Hq), shape(Hkv), torch.bfloat16)
+    n = torch.tensor(lens)
+    kw = dict(seqlens=n) if right else dict(left_paddings=S - n)
+    ref, ref_lse = O.padded_attention(q.float(), k.float(), v.float(), O.block_mask(Hq, S, num_kv_heads=Hkv, **pk), bs,
+                                      seq_dim=seq_dim, **kw)
+    mod = _module(Hq, S, dict(pk, num_kv_heads=Hkv), seq_dim=seq_dim, impl="sm100")
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+    kw = {a: t.cuda() for a, t in kw.items()}
+    for _ in range(2):
+        dirty = [torch.full_like(q, float("nan")), torch.full((B, Hq, S), float("nan"), device="cuda")]
+        del dirty      # back to the caching allocator, which hands the blocks out again
+        with torch.no_grad():
+            out, lse = mod(q, k, v, return_lse=True, **kw)
+        assert_out_close(out, ref)
+        assert_lse_close(lse, ref_lse)
+        assert ((ref == 0).all(-1) == (out.cpu() == 0).all(-1)).all()
+    own = torch.full_like(q, 7.0)
+    mod_out = _module(Hq, S, dict(pk, num_kv_heads=Hkv), seq_dim=seq_dim, impl="sm100", out=own)
+    with torch.no_grad():
+        mod_out(q, k, v, **kw)
+    pad = (ref == 0).all(-1)
+    assert (own.cpu()[pad] == 7.0).all() and torch.equal(own.cpu()[~pad], out.cpu()[~pad])
