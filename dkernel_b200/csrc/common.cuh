@@ -83,6 +83,7 @@ bool sm100_bwd_supported(const bsa_bwd_params* p, const char** why);
 int sm100_bwd(const bsa_bwd_params* p, cudaStream_t s);
 size_t decode_workspace_bytes(const bsa_decode_params* p);
 int decode_run(const bsa_decode_params* p, cudaStream_t s);
+int decode_packed_rows(const bsa_fwd_params* p, cudaStream_t s);
 int decode_run_static(const bsa_decode_params* p, cudaStream_t s);
 size_t decode_static_capacity();
 int merge_partials(const void* o_parts, const float* lse_parts, int P, int64_t rows, int d,

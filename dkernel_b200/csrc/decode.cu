@@ -33,7 +33,8 @@ constexpr int kRingBytes = 65536;        // K/V ring
 constexpr int kMinCtas = 3;              // resident CTAs per SM the kernel is built for
 constexpr int kConsumers = 4;            // consumer warps
 constexpr int kDecThreads = 32 * (kConsumers + 1);
-constexpr int kMaxTokens = 4096;         // tokens per CTA
+constexpr int kMaxTokens = 4096;         // tokens per CTA (a caller's blocks_per_split)
+constexpr int kMaxRowBlocks = 1024;      // blocks of one row in a packed batch (decode_packed_rows)
 constexpr float kDecRescale = 8.0f;      // log2 of how far a maximum may grow before O is rescaled
 
 template <typename T> struct MmaType;
@@ -113,7 +114,6 @@ template <int D, bool FP8> struct DecGeo {
   static constexpr int kTileBytes = kTok * D * (FP8 ? 1 : 2);
   static constexpr int kStageBytes = 2 * kTileBytes;
   static constexpr int kStages = kRingBytes / kStageBytes;
-  static constexpr int kMaxUnits = kMaxTokens / kTok;       // units per CTA
   static constexpr bool kSwizzle = !FP8 || D == 128;
   static_assert(kStages % kConsumers == 0, "a stage belongs to one consumer warp");
   // byte offset of 16-byte chunk `chunk` of token row `tok` in a tile
@@ -128,13 +128,13 @@ template <int D, bool FP8, int NT> struct DecodeSmem {
   alignas(16) uint16_t q[NT * 8][D];           // q heads of the group, zero rows behind them
   uint64_t full[DecGeo<D, FP8>::kStages];
   uint64_t empty[DecGeo<D, FP8>::kStages];
-  int n_units;                                 // units of this CTA
-  int unit_pos[DecGeo<D, FP8>::kMaxUnits];     // first position of each unit
   float wm[kConsumers][NT * 8];
   float wl[kConsumers][NT * 8];
+  int n_units;                                 // units of this CTA
+  int unit_pos[1];                             // first position of each unit: max_units entries
 };
-template <int D, bool FP8, int NT> constexpr size_t dec_smem() {
-  return 1024 + kRingBytes + sizeof(DecodeSmem<D, FP8, NT>);
+template <int D, bool FP8, int NT> size_t dec_smem(int max_units) {
+  return 1024 + kRingBytes + sizeof(DecodeSmem<D, FP8, NT>) + sizeof(int) * (size_t)max_units;
 }
 
 // four e4m3 bytes of a word -> two f16x2: (byte 0, byte 1) and (byte 2, byte 3); exact
@@ -159,7 +159,8 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
 template <typename T, int D, bool FP8, int NT>
 __global__ void __launch_bounds__(kDecThreads, FP8 && D == 128 && NT == 2 ? 2 : kMinCtas)   // 2: spills otherwise
 decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 tmV,
-              bsa_decode_params p, int nsplit, int* wait_status) {
+              bsa_decode_params p, int nsplit, int max_units, const int32_t* __restrict__ row_start,
+              const int32_t* __restrict__ row_end, int* wait_status) {
   using Geo = DecGeo<D, FP8>;
   constexpr int kStages = Geo::kStages, kTok = Geo::kTok;
   constexpr int kTileBytes = Geo::kTileBytes;
@@ -175,6 +176,13 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (*reinterpret_cast<volatile int*>(wait_status) != 0) return;  // an earlier wait gave up
   const int sp = blockIdx.x, b = blockIdx.z;
+  // Row of q, o and lse: the sequence's number, or (packed batch of chunks and decode tokens) the
+  // row of its single query token; sequences with another number of query tokens are not served here.
+  int qb = b;
+  if (row_start) {
+    qb = row_start[b];
+    if (row_end[b] - qb != 1) return;
+  }
   const int G = p.hq / p.hkv;
   const int GH = p.heads_per_cta;
   const int groups_per_kv = G / GH;
@@ -247,7 +255,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
             // positions grow with the entry index, so the units past the end form a tail
             const int pos = c * bs + s * kTok;
             const int u = (idx - want0) * subs + s;
-            if (pos < end_pos && u < Geo::kMaxUnits) {
+            if (pos < end_pos && u < max_units) {
               sm->unit_pos[u] = pos;
               ++valid_units;
             }
@@ -273,7 +281,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       const int r = i / (D / 8), c = i % (D / 8);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < GH) {
-        const T* src = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_sb + (int64_t)(h0 + r) * p.q_sh + c * 8;
+        const T* src = reinterpret_cast<const T*>(p.q) + (int64_t)qb * p.q_sb + (int64_t)(h0 + r) * p.q_sh + c * 8;
         if (q_vec) {
           v = *reinterpret_cast<const uint4*>(src);
         } else {
@@ -302,7 +310,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     for (int i = tid; i < GH * D; i += kDecThreads) {
       const int h = h0 + i / D, d = i % D;
       if (final_out) {
-        reinterpret_cast<T*>(p.o)[(int64_t)b * p.o_sb + (int64_t)h * p.o_sh + d] = Elem<T>::from_f(0.f);
+        reinterpret_cast<T*>(p.o)[(int64_t)qb * p.o_sb + (int64_t)h * p.o_sh + d] = Elem<T>::from_f(0.f);
       } else {
         p.ws[(((int64_t)b * p.hq + h) * nsplit + sp) * D + d] = 0.f;
       }
@@ -310,7 +318,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     for (int i = tid; i < GH; i += kDecThreads) {
       const int h = h0 + i;
       if (final_out) {
-        if (p.lse) p.lse[(int64_t)b * p.lse_sb + (int64_t)h * p.lse_sh] = -INFINITY;
+        if (p.lse) p.lse[(int64_t)qb * p.lse_sb + (int64_t)h * p.lse_sh] = -INFINITY;
       } else {
         p.ws[(int64_t)p.batch * p.hq * nsplit * D + ((int64_t)b * p.hq + h) * nsplit + sp] = -INFINITY;
       }
@@ -570,14 +578,14 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
     const int h = h0 + r;
     if (final_out) {
-      T* dst = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_sb + (int64_t)h * p.o_sh + d;
+      T* dst = reinterpret_cast<T*>(p.o) + (int64_t)qb * p.o_sb + (int64_t)h * p.o_sh + d;
       if (o_vec) {
         *reinterpret_cast<uint2*>(dst) = make_uint2(MmaType<T>::pack(acc.x, acc.y), MmaType<T>::pack(acc.z, acc.w));
       } else {
         dst[0] = Elem<T>::from_f(acc.x); dst[1] = Elem<T>::from_f(acc.y);
         dst[2] = Elem<T>::from_f(acc.z); dst[3] = Elem<T>::from_f(acc.w);
       }
-      if (d == 0 && p.lse) p.lse[(int64_t)b * p.lse_sb + (int64_t)h * p.lse_sh] = lse;
+      if (d == 0 && p.lse) p.lse[(int64_t)qb * p.lse_sb + (int64_t)h * p.lse_sh] = lse;
     } else {
       if (BSA_IN_BOUNDS(h < p.hq && sp < nsplit && d < D, wait_status, 822)) {
         float* dst = p.ws + (((int64_t)b * p.hq + h) * nsplit + sp) * D + d;
@@ -683,7 +691,8 @@ int decode_nsplit(const bsa_decode_params* p) {
 }
 
 template <typename T, int D, bool FP8, int NT>
-int launch_decode(const bsa_decode_params* p, cudaStream_t s) {
+int launch_decode(const bsa_decode_params* p, int nsplit, const int32_t* row_start, const int32_t* row_end,
+                  cudaStream_t s) {
   Tmap4 tmK, tmV;
   const bool bf16 = p->dtype == BSA_BF16;
   const int eb = FP8 ? 1 : 2;
@@ -695,17 +704,19 @@ int launch_decode(const bsa_decode_params* p, cudaStream_t s) {
   rc = make_tmap_4d(&tmV, p->v, eb, D, p->sk, p->hkv, p->batch, p->v_ss * eb, p->v_sh * eb,
                     p->v_sb * eb, box_d, Geo::kTok, Geo::kSwizzle, bf16);
   if (rc) return rc;
-  const int nsplit = decode_nsplit(p);
-  const size_t smem = dec_smem<D, FP8, NT>();
-  auto kern = decode_kernel<T, D, FP8, NT>;
-  BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int G = p->hq / p->hkv;
-  dim3 grid(nsplit, p->hkv * (G / p->heads_per_cta), p->batch);
   bsa_decode_params q = *p;
   q.blocks_per_split = decode_blocks_per_split(p);
+  const int max_units = q.blocks_per_split * (p->block_size / Geo::kTok);
+  const size_t smem = dec_smem<D, FP8, NT>(max_units);
+  auto kern = decode_kernel<T, D, FP8, NT>;
+  // one value for every call: host threads may launch this kernel with different sizes at the same time
+  BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)dec_smem<D, FP8, NT>(kMaxRowBlocks * 64 / Geo::kTok)));
+  const int G = p->hq / p->hkv;
+  dim3 grid(nsplit, p->hkv * (G / p->heads_per_cta), p->batch);
   int* status = wait_status_ptr();
   if (!status) return BSA_E_CUDA;
-  kern<<<grid, kDecThreads, smem, s>>>(tmK, tmV, q, nsplit, status);
+  kern<<<grid, kDecThreads, smem, s>>>(tmK, tmV, q, nsplit, max_units, row_start, row_end, status);
   rc = check_launch("decode_kernel");
   if (rc) return rc;
   if (nsplit > 1 && p->o) {
@@ -731,13 +742,15 @@ int launch_decode(const bsa_decode_params* p, cudaStream_t s) {
 }
 
 template <typename T>
-int launch_decode_t(const bsa_decode_params* p, bool fp8, cudaStream_t s) {
+int launch_decode_t(const bsa_decode_params* p, bool fp8, int nsplit, const int32_t* row_start,
+                    const int32_t* row_end, cudaStream_t s) {
+  auto go = [&](auto kernel) { return kernel(p, nsplit, row_start, row_end, s); };
   if (p->heads_per_cta > 8) {
-    if (fp8) return p->d == 128 ? launch_decode<T, 128, true, 2>(p, s) : launch_decode<T, 64, true, 2>(p, s);
-    return p->d == 128 ? launch_decode<T, 128, false, 2>(p, s) : launch_decode<T, 64, false, 2>(p, s);
+    if (fp8) return p->d == 128 ? go(launch_decode<T, 128, true, 2>) : go(launch_decode<T, 64, true, 2>);
+    return p->d == 128 ? go(launch_decode<T, 128, false, 2>) : go(launch_decode<T, 64, false, 2>);
   }
-  if (fp8) return p->d == 128 ? launch_decode<T, 128, true, 1>(p, s) : launch_decode<T, 64, true, 1>(p, s);
-  return p->d == 128 ? launch_decode<T, 128, false, 1>(p, s) : launch_decode<T, 64, false, 1>(p, s);
+  if (fp8) return p->d == 128 ? go(launch_decode<T, 128, true, 1>) : go(launch_decode<T, 64, true, 1>);
+  return p->d == 128 ? go(launch_decode<T, 128, false, 1>) : go(launch_decode<T, 64, false, 1>);
 }
 
 }  // namespace
@@ -777,8 +790,40 @@ int decode_run(const bsa_decode_params* p, cudaStream_t s) {
   }
   const int nsplit = decode_nsplit(p);
   BSA_CHECK_ARG((nsplit == 1 && p->o) || p->ws, "bsa_decode: workspace required for %d splits", nsplit);
-  if (p->dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(p, fp8, s);
-  return launch_decode_t<__half>(p, fp8, s);
+  if (p->dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(p, fp8, nsplit, nullptr, nullptr, s);
+  return launch_decode_t<__half>(p, fp8, nsplit, nullptr, nullptr, s);
+}
+
+// The sequences of a packed batch that have one query token.  A CTA walks a whole pattern row (there
+// is no scratch for partials); its list holds every block of the pattern's longest possible row.
+int decode_packed_rows(const bsa_fwd_params* f, cudaStream_t s) {
+  if (f->n_rows > kMaxRowBlocks && f->sk > kMaxRowBlocks * 64) {
+    set_error("bsa_fwd: a row of a packed batch has more than %d blocks", kMaxRowBlocks);
+    return BSA_E_TOOBIG;
+  }
+  bsa_decode_params p = {};
+  p.q = f->q; p.k = f->k; p.v = f->v; p.o = f->o; p.lse = f->lse;
+  p.q_sb = f->q_ss; p.q_sh = f->q_sh;
+  p.k_sb = f->k_sb; p.k_ss = f->k_ss; p.k_sh = f->k_sh;
+  p.v_sb = f->v_sb; p.v_ss = f->v_ss; p.v_sh = f->v_sh;
+  p.o_sb = f->o_ss; p.o_sh = f->o_sh;
+  p.lse_sb = 1; p.lse_sh = f->lse_sh;
+  p.batch = f->batch; p.hq = f->hq; p.hkv = f->hkv; p.d = f->d; p.sk = f->sk;
+  p.k_start = f->k_start; p.k_end = f->k_end;
+  p.crow = f->crow; p.col = f->col; p.crow_sh = f->crow_sh; p.col_sh = f->col_sh;
+  p.h_pat = f->h_pat; p.n_rows = f->n_rows; p.block_size = f->block_size;
+  // the heads of a CTA share a block list
+  const int G = f->hq / f->hkv;
+  p.heads_per_cta = 1;
+  if (f->h_pat != f->hq)
+    for (int c = 2; c <= G && c <= 16; ++c)
+      if (G % c == 0) p.heads_per_cta = c;
+  // columns ascend and a causal row sees no block past the sequence: its first cdiv(sk, 64) entries do
+  p.blocks_per_split = p.max_row_nnz = f->n_rows < cdiv_i(f->sk, 64) ? f->n_rows : cdiv_i(f->sk, 64);
+  p.dtype = f->dtype;
+  p.sm_scale = f->sm_scale;
+  if (p.dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(&p, false, 1, f->q_start, f->q_end, s);
+  return launch_decode_t<__half>(&p, false, 1, f->q_start, f->q_end, s);
 }
 
 int merge_partials(const void* o_parts, const float* lse_parts, int P, int64_t rows, int d,

@@ -453,3 +453,37 @@ def test_pad_rows_of_a_padded_batch_are_written(Hq, Hkv, S, D, bs, seq_dim, lens
         mod_out(q, k, v, **kw)
     pad = (ref == 0).all(-1)
     assert (own.cpu()[pad] == 7.0).all() and torch.equal(own.cpu()[~pad], out.cpu()[~pad])
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,dtype,user_pattern", [
+    (8, 2, 128, torch.bfloat16, False),     # four heads of a group in one decode CTA
+    (4, 4, 64, torch.float16, False),
+    (4, 2, 128, torch.bfloat16, True),      # a pattern per q head: one head per decode CTA
+    (24, 2, 64, torch.bfloat16, False),     # twelve heads: two column tiles
+    (4, 2, 96, torch.float16, False),       # not a head dim of the decode kernel
+])
+def test_packed_single_token_sequences_beside_chunks(Hq, Hkv, D, dtype, user_pattern):
+    """One packed call with empty sequences, single query tokens and chunks, more than 32 sequences: single
+    tokens run on the decode kernel, the rest on the prefill kernel, and every row of the output is written."""
+    from dkernel_b200 import SparseAttention
+    bs, S = 64, 4096
+    g = torch.Generator().manual_seed(4)
+    if user_pattern:
+        nb = S // bs
+        pat = torch.tril(torch.rand(Hq, nb, nb, generator=g) < 0.3) | torch.eye(nb, dtype=torch.bool)[None]
+        bm, mod = pat.numpy(), SparseAttention(bs, pat.to(torch.uint8).cuda(), impl="sm100")
+    else:
+        pk = dict(block_size=bs, local_blocks=3, vert_stride=4, num_kv_heads=Hkv)
+        bm, mod = O.block_mask(Hq, S, **pk), _module(Hq, S, pk, impl="sm100")
+    q_lens = [1, 130, 0, 1, 64, 1] + [1] * 30 + [63, 1]
+    k_lens = [1, 130, 0, 64, 128, 65] + [1 + int(x) for x in torch.randint(0, 900, (30,), generator=g)] + [191, 4096]
+    cu_q = torch.tensor(np.cumsum([0] + q_lens), dtype=torch.int32)
+    cu_k = torch.tensor(np.cumsum([0] + k_lens), dtype=torch.int32)
+    q, k, v = seeded_qkv(81, (sum(q_lens), Hq, D), (sum(k_lens), Hkv, D), dtype)
+    ref, ref_lse = O.varlen_attention(q.float(), k.float(), v.float(), cu_k, bm, bs, cu_seqlens_q=cu_q)
+    dirty = torch.full_like(q, float("nan")).cuda()
+    del dirty
+    with torch.no_grad():
+        out, lse = mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda(), return_lse=True)
+    assert_out_close(out, ref)
+    assert_lse_close(lse, ref_lse)
