@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 import torch
 
@@ -27,6 +28,15 @@ class LocalStrideParams(C.Structure):
         "head_sliding_step", "head_sliding_offset", "causal", "absolute_vert")]
 
 
+def _packer(cls):
+    """struct.Struct with the members of a ctypes structure, in order: one pack() of all values costs a
+    tenth of setting the fields one by one (they are most of the host time of a small call)."""
+    code = {_vp: "P", _i64: "q", _i32: "i", _f32: "f"}
+    s = struct.Struct("@" + "".join(code[t] for _, t in cls._fields_) + "0P")
+    assert s.size == C.sizeof(cls)
+    return s
+
+
 class FwdParams(C.Structure):
     _fields_ = (
         [(n, _vp) for n in ("q", "k", "v", "o", "lse")]
@@ -39,6 +49,9 @@ class FwdParams(C.Structure):
         + [("sm_scale", _f32), ("col_bits", _vp), ("col_bits_sh", _i64), ("fine_block", _i32),
            ("tile_counter", _vp)]
     )
+
+
+FWD_PACK = _packer(FwdParams)
 
 
 class BwdParams(C.Structure):
@@ -67,6 +80,9 @@ class DecodeParams(C.Structure):
         + [("sm_scale", _f32), ("ws", _vp), ("k_blk_mod", _i32), ("k_blk_rem", _i32),
            ("kv_dtype", _i32), ("k_scale", _f32), ("v_scale", _f32)]
     )
+
+
+DECODE_PACK = _packer(DecodeParams)
 
 
 class XchgParams(C.Structure):
@@ -179,6 +195,18 @@ def dtype_code(dt: torch.dtype) -> int:
 
 def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
+
+
+def launch(fn, params, device_index: int, what: str) -> None:
+    """fn(&params, stream) on the device's current stream, with that device current."""
+    if device_index not in _armed:
+        _arm_mirror(device_index)
+    stream = torch._C._cuda_getCurrentRawStream(device_index)
+    if torch._C._cuda_getDevice() == device_index:
+        check(fn(C.byref(params), stream), what)
+    else:
+        with torch.cuda.device(device_index):
+            check(fn(C.byref(params), stream), what)
 
 
 def stream_of(t: torch.Tensor) -> int:

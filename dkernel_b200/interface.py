@@ -129,8 +129,9 @@ class SparseAttention(torch.nn.Module):
         self._plan_cache = None
 
     def _plan(self) -> _Plan:
-        p = self._plan_cache
-        if p is None or p.crow.data_ptr() != self._blk_crow.data_ptr() or p.crow.device != self._blk_crow.device:
+        p, crow = self._plan_cache, self._buffers["_blk_crow"]
+        if p is None or (p.crow is not crow and
+                         (p.crow.data_ptr() != crow.data_ptr() or p.crow.device != crow.device)):
             p = _Plan(self._blk_crow, self._blk_col, self.layout_csc_ccol, self.layout_csc_row,
                       self.block_size, self._max_row_nnz)
             self._plan_cache = p
@@ -159,14 +160,12 @@ class SparseAttention(torch.nn.Module):
                       "left_paddings": left_paddings,
                       "seqlens": seqlens,
                       "kv_scales": kv_scales}
-        kwargs = copy.copy(self.kwargs)
-        kwargs["return_lse"] = return_lse
-        kwargs["split_qkv"] = split_qkv
-        kwargs["_plan"] = self._plan()
+        kwargs = {**self.kwargs, "return_lse": return_lse, "split_qkv": split_qkv, "_plan": self._plan()}
+        buf = self._buffers
         output, lse = _sparse_attention.apply(
             q, k, v, sm_scale,
-            (self.layout_csr_crow, self.layout_csr_col, self.block_m, self.block_n),
-            (self.layout_csc_ccol, self.layout_csc_row, self.block_m2, self.block_n2),
+            (buf["layout_csr_crow"], buf["layout_csr_col"], self.block_m, self.block_n),
+            (buf["layout_csc_ccol"], buf["layout_csc_row"], self.block_m2, self.block_n2),
             self.seq_dim, inf_kwargs, kwargs)
         if return_lse:
             return output, lse

@@ -27,20 +27,30 @@ def _last_dim_contig(t: Tensor) -> Tensor:
 def _tma_friendly(t: Tensor) -> Tensor:
     """Tensor-map requirements of the tcgen05 / decode kernels: 16-byte aligned
     base and strides that are multiples of 16 bytes.  Anything else is copied."""
-    t = _last_dim_contig(t)
-    if t.element_size() > 2:
+    st = t.stride()
+    if st[-1] != 1:
+        t = t.contiguous()
+        st = t.stride()
+    size = t.element_size()
+    if size > 2:
         return t
-    per16 = 16 // t.element_size()
-    ok = t.data_ptr() % 16 == 0 and all(s % per16 == 0 for s in t.stride()[:-1])
-    return t if ok else t.contiguous()
+    bits = t.data_ptr()
+    for s in st[:-1]:
+        bits |= s * size
+    return t.contiguous() if bits & 15 else t
+
+
+def _empty_like(t: Tensor) -> Tensor:
+    """Uninitialised and contiguous, whatever the strides of ``t``."""
+    return torch.empty_like(t, memory_format=torch.contiguous_format)
 
 
 def _strides_bsh(t: Tensor, seq_dim: Optional[int]) -> Tuple[int, int, int]:
     """(batch, seq, head) element strides of a 4-D (seq_dim 1 or 2) or packed 3-D tensor."""
-    if t.dim() == 3:
-        return 0, t.stride(0), t.stride(1)
-    hdim = 3 - seq_dim
-    return t.stride(0), t.stride(seq_dim), t.stride(hdim)
+    st = t.stride()
+    if len(st) == 3:
+        return 0, st[0], st[1]
+    return st[0], st[seq_dim], st[3 - seq_dim]
 
 
 class _Plan:
@@ -62,6 +72,22 @@ class _Plan:
         self._cyclic_nnz: Dict[Tuple[int, int], int] = {}
         self._max_head_nnz: Optional[int] = None
         self._csc_csr: Optional[Tensor] = None
+        self._dims: Optional[Tuple[int, int, int, int, int]] = None
+
+    def layout_dims(self) -> Tuple[int, int, int, int, int]:
+        """(crow head stride, col head stride, pattern heads, rows, block size) as the kernels take them."""
+        if self._dims is None:
+            heads, width = self.crow.shape
+            strides = (self.crow.stride(0), self.col.stride(0)) if heads > 1 else (0, 0)
+            self._dims = (*strides, heads, width - 1, self.block_size)
+        return self._dims
+
+    def bits_args(self) -> Tuple[int, int, int]:
+        """(col_bits, its head stride, fine block size); zeros where the pattern's blocks are the kernel's."""
+        cb = self.col_bits
+        if cb is None:
+            return 0, 0, 0
+        return cb.data_ptr(), cb.stride(0) if cb.size(0) > 1 else 0, self.fine_block
 
     def max_row_nnz_cyclic(self, mod: int, rem: int) -> int:
         """Longest pattern row when only the blocks congruent to ``rem`` modulo ``mod`` count
@@ -226,51 +252,46 @@ class _Plan:
 
 
 def _fill_layout(p, plan: _Plan) -> None:
-    p.crow, p.col = _lib.ptr(plan.crow), _lib.ptr(plan.col)
-    p.crow_sh = plan.crow.stride(0) if plan.crow.size(0) > 1 else 0
-    p.col_sh = plan.col.stride(0) if plan.col.size(0) > 1 else 0
-    p.h_pat = plan.crow.size(0)
-    p.n_rows = plan.crow.size(1) - 1
-    p.block_size = plan.block_size
+    """Sets the layout fields of forward or decode parameters."""
+    p.crow, p.col = plan.crow.data_ptr(), plan.col.data_ptr()
+    p.crow_sh, p.col_sh, p.h_pat, p.n_rows, p.block_size = plan.layout_dims()
     if hasattr(p, "fine_block"):
-        cb = getattr(plan, "col_bits", None)
-        p.col_bits = _lib.ptr(cb)
-        p.col_bits_sh = cb.stride(0) if cb is not None and cb.size(0) > 1 else 0
-        p.fine_block = plan.fine_block if cb is not None else 0
+        p.col_bits, p.col_bits_sh, p.fine_block = plan.bits_args()
 
 
 def _fwd_params(q, k, v, o, lse, seq_dim, plan: _Plan, sm_scale, causal, row_mode,
                 q_start=None, q_end=None, k_start=None, k_end=None, total_q=0, impl=0, kernel_plan=True):
-    p = _lib.FwdParams()
     own_plan = plan
     if impl != _lib.IMPL_GENERIC and kernel_plan:
         plan = plan.for_kernels(q)
-    p.q, p.k, p.v, p.o, p.lse = _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse)
-    p.q_sb, p.q_ss, p.q_sh = _strides_bsh(q, seq_dim)
-    p.k_sb, p.k_ss, p.k_sh = _strides_bsh(k, seq_dim)
-    p.v_sb, p.v_ss, p.v_sh = _strides_bsh(v, seq_dim)
-    p.o_sb, p.o_ss, p.o_sh = _strides_bsh(o, seq_dim)
-    if q.dim() == 3:
-        p.batch = q_start.numel()
-        p.hq, p.hkv, p.d = q.size(1), k.size(1), q.size(2)
-        p.sq, p.sk = q.size(0), k.size(0)
+    q_sb, q_ss, q_sh = _strides_bsh(q, seq_dim)
+    k_sb, k_ss, k_sh = _strides_bsh(k, seq_dim)
+    v_sb, v_ss, v_sh = _strides_bsh(v, seq_dim)
+    o_sb, o_ss, o_sh = _strides_bsh(o, seq_dim)
+    lse_ptr = lse_sb = lse_sh = 0
+    qs, ks = q.shape, k.shape
+    if len(qs) == 3:
+        batch = q_start.numel()
+        sq, hq, d = qs
+        sk, hkv = ks[0], ks[1]
         if lse is not None:          # (Hq, total tokens)
-            p.lse_sb, p.lse_sh = 0, lse.stride(0)
+            lse_ptr, lse_sh = lse.data_ptr(), lse.stride(0)
     else:
-        hdim = 3 - seq_dim
-        p.batch, p.hq, p.hkv, p.d = q.size(0), q.size(hdim), k.size(hdim), q.size(3)
-        p.sq, p.sk = q.size(seq_dim), k.size(seq_dim)
+        batch, d = qs[0], qs[3]
+        sq, hq = qs[seq_dim], qs[3 - seq_dim]
+        sk, hkv = ks[seq_dim], ks[3 - seq_dim]
         if lse is not None:          # (B, Hq, Sq)
-            p.lse_sb, p.lse_sh = lse.stride(0), lse.stride(1)
-    p.total_q = total_q
-    p.q_start, p.q_end = _lib.ptr(q_start), _lib.ptr(q_end)
-    p.k_start, p.k_end = _lib.ptr(k_start), _lib.ptr(k_end)
-    _fill_layout(p, plan)
-    p.causal = 1 if causal else 0
-    p.row_mode = row_mode
-    p.dtype = _lib.dtype_code(q.dtype)
-    p.impl = impl
-    p.sm_scale = float(sm_scale)
+            lse_ptr = lse.data_ptr()
+            lse_sb, lse_sh, _ = lse.stride()
+    crow_sh, col_sh, h_pat, n_rows, block_size = plan.layout_dims()
+    p = _lib.FwdParams.from_buffer_copy(_lib.FWD_PACK.pack(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse_ptr,
+        q_sb, q_ss, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, lse_sb, lse_sh,
+        batch, hq, hkv, d, sq, sk, total_q,
+        _lib.ptr(q_start), _lib.ptr(q_end), _lib.ptr(k_start), _lib.ptr(k_end),
+        plan.crow.data_ptr(), plan.col.data_ptr(), crow_sh, col_sh,
+        h_pat, n_rows, block_size, 1 if causal else 0, row_mode, _lib.dtype_code(q.dtype), impl,
+        float(sm_scale), *plan.bits_args(), 0))      # last: tile_counter
     if plan.fine_block and impl == _lib.IMPL_AUTO and _lib.lib().bsa_fwd_why_not_sm100(C.byref(p)):
         # the coarsened form is only read by the tensor-core kernel: hand the pattern's own layout on
         _fill_layout(p, own_plan)
@@ -302,22 +323,23 @@ def _launch_fwd(p, q: Tensor) -> None:
             # counter (zeroed on this stream; a memset node under graph capture)
             counter = torch.zeros(1, dtype=torch.int32, device=q.device)
             p.tile_counter = _lib.ptr(counter)
-    with torch.cuda.device(q.device):
-        _lib.check(lib.bsa_fwd(C.byref(p), _lib.stream_of(q)), "bsa_fwd")
+    _lib.launch(lib.bsa_fwd, p, q.get_device(), "bsa_fwd")
 
 
 _FP8 = getattr(torch, "float8_e4m3fn", None)
 
 
 def _check_inputs(q: Tensor, k: Tensor, v: Tensor) -> None:
-    for n, t in (("q", q), ("k", k), ("v", v)):
-        _lib.require_cuda(t, n)
-    if _FP8 is not None and k.dtype == _FP8 and v.dtype == _FP8:
-        assert q.dtype in (torch.float16, torch.bfloat16), "an e4m3 K/V cache needs f16/bf16 queries"
+    if not (q.is_cuda and k.is_cuda and v.is_cuda):
+        for n, t in (("q", q), ("k", k), ("v", v)):
+            _lib.require_cuda(t, n)
+    qt, kt, vt = q.dtype, k.dtype, v.dtype
+    if _FP8 is not None and kt == _FP8 and vt == _FP8:
+        assert qt in (torch.float16, torch.bfloat16), "an e4m3 K/V cache needs f16/bf16 queries"
     else:
-        assert q.dtype == k.dtype == v.dtype, f"q/k/v dtypes differ: {q.dtype}, {k.dtype}, {v.dtype}"
-    assert q.device == k.device == v.device
-    _lib.dtype_code(q.dtype)
+        assert qt == kt == vt, f"q/k/v dtypes differ: {qt}, {kt}, {vt}"
+    assert q.get_device() == k.get_device() == v.get_device()
+    _lib.dtype_code(qt)
 
 
 _IMPL_NAMES = {None: _lib.IMPL_AUTO, "auto": _lib.IMPL_AUTO, "generic": _lib.IMPL_GENERIC,
@@ -336,8 +358,8 @@ def _fp8_kv_scales(q: Tensor, k: Tensor, kv_scales) -> Optional[Tuple[float, flo
 
 
 def _decode_eligible(q: Tensor, plan: _Plan, impl: int) -> bool:
-    return (impl != _lib.IMPL_GENERIC and q.dtype in (torch.float16, torch.bfloat16)
-            and q.size(-1) in (64, 128) and plan.block_size in (64, 128))
+    return (impl != _lib.IMPL_GENERIC and plan.block_size in (64, 128) and q.shape[-1] in (64, 128)
+            and q.dtype in (torch.float16, torch.bfloat16))
 
 
 def _pick_heads_per_cta(g: int) -> int:
@@ -353,26 +375,27 @@ def decode(q: Tensor, k: Tensor, v: Tensor, plan: _Plan, sm_scale: float, *, seq
            out: Optional[Tensor] = None, blocks_per_split: int = 0,
            workspace: Optional[Tensor] = None, lse_out: Optional[Tensor] = None,
            k_blk: Optional[Tuple[int, int]] = None, partials_only: bool = False,
-           kv_scales: Optional[Tuple[float, float]] = None) -> Tuple[Tensor, Tensor]:
+           kv_scales: Optional[Tuple[float, float]] = None,
+           need_lse: bool = True) -> Tuple[Tensor, Optional[Tensor]]:
     """One query token per sequence (split-KV decode kernel).
 
     q: (B,1,Hq,D)/(B,Hq,1,D) or packed (B,Hq,D); k, v: 4-D with the module's
     seq_dim, or packed (T,Hkv,D) with ``k_start``/``k_end`` = cu_seqlens slices.
     ``k_pos0``/``k_total`` describe a contiguous KV shard, ``k_blk = (W, r)`` with ``k_total`` a
     block-cyclic one (see include/bsa.h).
-    Returns (out shaped like q, lse fp32 (B,Hq)); with ``partials_only`` the split-KV partials
+    Returns (out shaped like q, lse fp32 (B,Hq), or None without ``need_lse``); with ``partials_only`` the split-KV partials
     stay unmerged and (o_parts fp32 (B*Hq, splits, D), lse_parts fp32 (B*Hq, splits)) are returned
     (views of one workspace tensor) for a consumer that merges them itself."""
     lib = _lib.lib()
     q = _last_dim_contig(q)     # before the strides are read: a copy has its own
     if q.dim() == 4:
-        B = q.size(0)
         hdim = 3 - seq_dim
-        hq, d = q.size(hdim), q.size(3)
-        q_sb, q_sh = q.stride(0), q.stride(hdim)
+        shape, st = q.shape, q.stride()
+        B, hq, d = shape[0], shape[hdim], shape[3]
+        q_sb, q_sh = st[0], st[hdim]
     else:
         B, hq, d = q.shape
-        q_sb, q_sh = q.stride(0), q.stride(1)
+        q_sb, q_sh, _ = q.stride()
     if partials_only:
         o, o_sh, lse, lse_sh = None, d, None, 1
     elif out is not None and out.dim() == 2:
@@ -380,7 +403,7 @@ def decode(q: Tensor, k: Tensor, v: Tensor, plan: _Plan, sm_scale: float, *, seq
         assert out.shape == (B * hq, d) and out.stride(1) == 1 and out.dtype == q.dtype
         o, o_sh = out, out.stride(0)
     else:
-        o = out if out is not None else torch.empty(q.shape, dtype=q.dtype, device=q.device)
+        o = out if out is not None else _empty_like(q)
         assert o.is_contiguous(), "decode output must be contiguous"
         o_sh = d
     if partials_only:
@@ -388,47 +411,43 @@ def decode(q: Tensor, k: Tensor, v: Tensor, plan: _Plan, sm_scale: float, *, seq
     elif lse_out is not None:
         assert lse_out.dtype == torch.float32 and lse_out.numel() == B * hq and lse_out.dim() == 1
         lse, lse_sh = lse_out, lse_out.stride(0)
+    elif need_lse:
+        lse, lse_sh = q.new_empty((B, hq), dtype=torch.float32), 1
     else:
-        lse, lse_sh = torch.empty((B, hq), dtype=torch.float32, device=q.device), 1
-    p = _lib.DecodeParams()
+        lse, lse_sh = None, 1
     k = _tma_friendly(k)
     v = _tma_friendly(v)
-    p.q, p.k, p.v, p.o, p.lse = _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse)
-    p.q_sb, p.q_sh = q_sb, q_sh
-    p.k_sb, p.k_ss, p.k_sh = _strides_bsh(k, seq_dim)
-    p.v_sb, p.v_ss, p.v_sh = _strides_bsh(v, seq_dim)
-    p.o_sb, p.o_sh = hq * o_sh, o_sh
-    p.lse_sb, p.lse_sh = hq * lse_sh, lse_sh
-    if k.dim() == 3:
-        hkv, sk = k.size(1), k.size(0)
-    else:
-        hkv, sk = k.size(3 - seq_dim), k.size(seq_dim)
-    p.batch, p.hq, p.hkv, p.d, p.sk = B, hq, hkv, d, sk
-    p.k_start, p.k_end = _lib.ptr(k_start), _lib.ptr(k_end)
-    p.k_pos0, p.k_total = _lib.ptr(k_pos0), _lib.ptr(k_total)
-    _fill_layout(p, plan)
-    g = hq // hkv
-    p.heads_per_cta = _pick_heads_per_cta(g) if plan.heads_shared_in_group(hq, hkv) else 1
-    p.blocks_per_split = blocks_per_split if blocks_per_split > 0 else 0   # 0: the library picks
-    p.max_row_nnz = plan.max_row_nnz
+    k_sb, k_ss, k_sh = _strides_bsh(k, seq_dim)
+    v_sb, v_ss, v_sh = _strides_bsh(v, seq_dim)
+    ks = k.shape
+    hkv, sk = (ks[1], ks[0]) if len(ks) == 3 else (ks[3 - seq_dim], ks[seq_dim])
+    crow_sh, col_sh, h_pat, n_rows, block_size = plan.layout_dims()
+    heads_per_cta = _pick_heads_per_cta(hq // hkv) if plan.heads_shared_in_group(hq, hkv) else 1
+    max_row_nnz, blk_mod, blk_rem = plan.max_row_nnz, 0, 0
     if k_blk is not None and k_blk[0] > 1:
-        p.k_blk_mod, p.k_blk_rem = k_blk
-        p.max_row_nnz = plan.max_row_nnz_cyclic(*k_blk)
-    p.dtype = _lib.dtype_code(q.dtype)
-    p.sm_scale = float(sm_scale)
+        blk_mod, blk_rem = k_blk
+        max_row_nnz = plan.max_row_nnz_cyclic(*k_blk)
+    kv_dtype, k_scale, v_scale = 0, 0.0, 0.0
     if kv_scales is not None:       # e4m3 K/V cache
         assert k.dtype == _FP8 and v.dtype == _FP8
-        p.kv_dtype, p.k_scale, p.v_scale = _lib.BSA_F8E4M3, float(kv_scales[0]), float(kv_scales[1])
+        kv_dtype, k_scale, v_scale = _lib.BSA_F8E4M3, float(kv_scales[0]), float(kv_scales[1])
+    p = _lib.DecodeParams.from_buffer_copy(_lib.DECODE_PACK.pack(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr(o), _lib.ptr(lse),
+        q_sb, q_sh, k_sb, k_ss, k_sh, v_sb, v_ss, v_sh, hq * o_sh, o_sh, hq * lse_sh, lse_sh,
+        B, hq, hkv, d, sk,
+        _lib.ptr(k_start), _lib.ptr(k_end), _lib.ptr(k_pos0), _lib.ptr(k_total),
+        plan.crow.data_ptr(), plan.col.data_ptr(), crow_sh, col_sh,
+        h_pat, n_rows, block_size, heads_per_cta, max(blocks_per_split, 0), max_row_nnz,   # 0 blocks: the library picks
+        _lib.dtype_code(q.dtype), float(sm_scale), 0, blk_mod, blk_rem, kv_dtype, k_scale, v_scale))
     need = lib.bsa_decode_workspace_bytes(C.byref(p))
     ws = None
     if need:
         if workspace is not None and workspace.numel() * workspace.element_size() >= need:
             ws = workspace
         else:
-            ws = torch.empty((need + 3) // 4, dtype=torch.float32, device=q.device)
-    p.ws = _lib.ptr(ws)
-    with torch.cuda.device(q.device):
-        _lib.check(lib.bsa_decode(C.byref(p), _lib.stream_of(q)), "bsa_decode")
+            ws = q.new_empty((need + 3) // 4, dtype=torch.float32)
+        p.ws = ws.data_ptr()
+    _lib.launch(lib.bsa_decode, p, q.get_device(), "bsa_decode")
     if partials_only:
         rows = B * hq
         nsplit = need // (4 * rows * (d + 1))
@@ -465,13 +484,13 @@ def _varlen(q, k, v, cu_seqlens_k, cu_seqlens_q, sm_scale, plan, causal, out, im
     fp8 = _fp8_kv_scales(q, k, kv_scales)
     if decoding and _decode_eligible(q, plan, impl):
         o, lse = decode(q, k, v, plan, sm_scale, seq_dim=None, k_start=cu_k[:-1], k_end=cu_k[1:],
-                        out=out, kv_scales=fp8)
+                        out=out, kv_scales=fp8, need_lse=return_lse)
         return o, (lse.transpose(0, 1) if return_lse else None)
     assert fp8 is None, "an e4m3 K/V cache is only read by the decode kernel (one query token per sequence)"
     if decoding:
         cu_q = torch.arange(0, batch + 1, dtype=torch.int32, device=q.device)
     q, k, v = _tma_friendly(q), _tma_friendly(k), _tma_friendly(v)
-    o = out if out is not None else torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    o = out if out is not None else _empty_like(q)
     lse = torch.full((q.size(1), q.size(0)), float("-inf"), dtype=torch.float32, device=q.device) \
         if return_lse else None
     p = _fwd_params(q, k, v, o, lse, None, plan, sm_scale, causal, _lib.ROWS_BY_POSITION,
@@ -486,12 +505,13 @@ def _padded(q, k, v, sm_scale, plan, left_paddings, seqlens, seq_dim, max_seqlen
     rows of the output are zero, positions are re-based to the first real token."""
     assert seq_dim in (1, 2)
     hdim = 3 - seq_dim
-    batches = q.size(0)
-    q_len, k_len = q.size(seq_dim), k.size(seq_dim)
-    assert q.dim() == k.dim() == v.dim() == 4
-    assert q.size(hdim) % k.size(hdim) == 0
-    assert q.size(0) == k.size(0) and q.size(3) == k.size(3)
-    assert k.shape == v.shape
+    qs, ks = q.shape, k.shape
+    assert len(qs) == len(ks) == 4 and v.dim() == 4
+    batches = qs[0]
+    q_len, k_len = qs[seq_dim], ks[seq_dim]
+    assert qs[hdim] % ks[hdim] == 0
+    assert batches == ks[0] and qs[3] == ks[3]
+    assert ks == v.shape
     assert q_len == 1 or q_len == k_len, \
         (f"q length can only 1 for decoding or the same as k length for prefilling, "
          f"but got {q_len=}, {k_len=}.")
@@ -500,7 +520,7 @@ def _padded(q, k, v, sm_scale, plan, left_paddings, seqlens, seq_dim, max_seqlen
     dev = q.device
     if left_paddings is not None:
         assert left_paddings.shape == (batches,)
-        k_starts = left_paddings.to(dev, dtype=torch.int32).contiguous()
+        k_starts = left_paddings.to(device=q.device, dtype=torch.int32).contiguous()
     else:
         k_starts = torch.zeros((batches,), dtype=torch.int32, device=dev)
     if seqlens is not None:
@@ -510,7 +530,7 @@ def _padded(q, k, v, sm_scale, plan, left_paddings, seqlens, seq_dim, max_seqlen
     fp8 = _fp8_kv_scales(q, k, kv_scales)
     if q_len == 1 and _decode_eligible(q, plan, impl):
         o, lse = decode(q, k, v, plan, sm_scale, seq_dim=seq_dim, k_start=k_starts, k_end=k_ends, out=out,
-                        kv_scales=fp8)
+                        kv_scales=fp8, need_lse=return_lse)
         return o, (lse.unsqueeze(-1) if return_lse else None)
     assert fp8 is None, "an e4m3 K/V cache is only read by the decode kernel (one query token per sequence)"
     if k_ends is None:
@@ -521,8 +541,8 @@ def _padded(q, k, v, sm_scale, plan, left_paddings, seqlens, seq_dim, max_seqlen
     else:
         q_starts, q_ends = k_starts, k_ends
     q, k, v = _tma_friendly(q), _tma_friendly(k), _tma_friendly(v)
-    o = out if out is not None else torch.empty(q.shape, dtype=q.dtype, device=dev)
-    lse = torch.empty((batches, q.size(hdim), q_len), dtype=torch.float32, device=dev) if return_lse else None
+    o = out if out is not None else _empty_like(q)
+    lse = q.new_empty((batches, qs[hdim], q_len), dtype=torch.float32) if return_lse else None
     # pad rows: the tensor-core kernel writes them; a caller's own output keeps what it holds there
     p = _fwd_params(q, k, v, o, lse, seq_dim, plan, sm_scale, causal,
                     _lib.ROWS_BY_POSITION_ZERO_PADS if out is None else _lib.ROWS_BY_POSITION,
@@ -544,10 +564,11 @@ def _train_forward(ctx, q, k, v, sm_scale, plan, seq_dim, causal, out, impl, nee
     (:435-440)."""
     assert seq_dim in (1, 2)
     hdim = 3 - seq_dim
-    assert q.shape[-1] == k.shape[-1] == v.shape[-1]
-    assert k.shape[seq_dim] == v.shape[seq_dim]
-    qlen, klen = q.size(seq_dim), k.size(seq_dim)
-    hq, hkv = q.size(hdim), k.size(hdim)
+    qs, ks, vs = q.shape, k.shape, v.shape
+    assert qs[-1] == ks[-1] == vs[-1]
+    assert ks[seq_dim] == vs[seq_dim]
+    qlen, klen = qs[seq_dim], ks[seq_dim]
+    hq, hkv = qs[hdim], ks[hdim]
     assert hq % hkv == 0
     dev = q.device
     fp8 = _fp8_kv_scales(q, k, kv_scales)
@@ -561,8 +582,8 @@ def _train_forward(ctx, q, k, v, sm_scale, plan, seq_dim, causal, out, impl, nee
         "a single query token against a longer key sequence is an inference-only call (inference=True)"
     row_mode = _lib.ROWS_BY_POSITION if qlen == 1 else _lib.ROWS_BY_TILE
     q, k, v = _tma_friendly(q), _tma_friendly(k), _tma_friendly(v)
-    o = out if out is not None else torch.empty(q.shape, dtype=q.dtype, device=dev)
-    lse = torch.empty((q.size(0), hq, qlen), dtype=torch.float32, device=dev) if need_lse else None
+    o = out if out is not None else _empty_like(q)
+    lse = q.new_empty((qs[0], hq, qlen), dtype=torch.float32) if need_lse else None
     p = _fwd_params(q, k, v, o, lse, seq_dim, plan, sm_scale, causal, row_mode, impl=impl)
     _launch_fwd(p, q)
     if ctx is not None and not inference:
@@ -632,8 +653,7 @@ def _backward(ctx, do: Tensor, dlse: Optional[Tensor], dq=None, dk=None, dv=None
             bp.ds_ws = _lib.ptr(ds_ws)
             bp.ds_tiles_per_head = tiles
             bp.csc_csr = _lib.ptr(plan.csc_to_csr())
-    with torch.cuda.device(q.device):
-        _lib.check(_lib.lib().bsa_bwd(C.byref(bp), _lib.stream_of(q)), "bsa_bwd")
+    _lib.launch(_lib.lib().bsa_bwd, bp, q.get_device(), "bsa_bwd")
     return dq, dk, dv
 
 
@@ -666,16 +686,17 @@ class _sparse_attention(torch.autograd.Function):
         ctx.bwd_impl = _IMPL_NAMES[kwargs.get("bwd_impl", "generic" if kwargs.get("impl") == "generic"
                                               else None)]
 
-        hdim = 3 - (seq_dim or 1) if q.dim() == 4 else 1
-        n_pat = layout_csr[0].size(0)
-        assert n_pat in [1, k.size(hdim), q.size(hdim)], \
-            (f"Input (q, k) have ({q.size(hdim)}, {k.size(hdim)}) heads"
+        qs, ks = q.shape, k.shape
+        hdim = 3 - (seq_dim or 1) if len(qs) == 4 else 1
+        n_pat = layout_csr[0].shape[0]
+        assert n_pat == 1 or n_pat == ks[hdim] or n_pat == qs[hdim], \
+            (f"Input (q, k) have ({qs[hdim]}, {ks[hdim]}) heads"
              f"but the number of heads in the sparse pattern is {n_pat}")
-        sm_scale = sm_scale or 1. / math.sqrt(float(q.size(-1)))
-        assert q.dim() in (3, 4)
+        sm_scale = sm_scale or 1. / math.sqrt(float(qs[-1]))
+        assert len(qs) in (3, 4)
 
         needs_grad = q.requires_grad or k.requires_grad or v.requires_grad
-        if q.dim() == 3:
+        if len(qs) == 3:
             assert inf_kwargs.get("cu_seqlen_k", None) is not None
             ctx.support_backward = False
             ctx.message = "Currently does not suppoort variable length inputs. WIP."
@@ -683,8 +704,8 @@ class _sparse_attention(torch.autograd.Function):
                                   sm_scale, plan, causal, out, impl, return_lse,
                                   kv_scales=inf_kwargs.get("kv_scales"))
         else:
-            assert k.size(seq_dim) <= max_seqlen, \
-                (f"Input length {k.size(seq_dim)} is larger "
+            assert ks[seq_dim] <= max_seqlen, \
+                (f"Input length {ks[seq_dim]} is larger "
                  f"than the maximum length allowed ({max_seqlen})")
             left_paddings = inf_kwargs.get("left_paddings", None)
             seqlens = inf_kwargs.get("seqlens", None)
