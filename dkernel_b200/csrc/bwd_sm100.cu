@@ -138,6 +138,29 @@ __global__ void bwd_delta_vec_kernel(bsa_bwd_params bp) {
   }
 }
 
+// ------------------------------------------------------------------ order of the tiles
+// Which (tile rank, sequence and head) a CTA of the one-dimensional grids works on.  Ranks go from the
+// longest tile to the shortest.  Head after head, a launch would end with the long tiles of its last
+// head; so the last `tail` heads, about two rounds of CTAs, take turns at each rank.  (4 x 1500 tokens,
+// 16/4 heads, D 64, where the 192 dK/dV CTAs are 1.3 rounds: dK/dV 171 -> 115 us, dQ behind it done
+// 50 us earlier.)  The heads in front of them stay one by one: turns over all heads cost more in
+// L2 misses than the tail gives (2 x 8192 tokens, 32 heads, D 128: 2.498 -> 2.533 ms a step).
+struct TileOrder { int n_ranks, n_heads, tail; };
+__device__ __forceinline__ void tile_of_cta(const TileOrder& o, int* rank, int* head) {
+  const int id = (int)blockIdx.x, front = (o.n_heads - o.tail) * o.n_ranks;
+  if (id < front) {
+    *head = id / o.n_ranks;
+    *rank = id % o.n_ranks;
+  } else {
+    *rank = (id - front) / o.tail;
+    *head = o.n_heads - o.tail + (id - front) % o.tail;
+  }
+}
+inline TileOrder tile_order(int n_ranks, int n_heads, int ctas_per_sm) {
+  const int tail = cdiv_i(2 * 148 * ctas_per_sm, n_ranks);
+  return {n_ranks, n_heads, tail < n_heads ? tail : n_heads};
+}
+
 // ------------------------------------------------------------------ shared list builder
 // Ordered union of two sets of block indices given as bitmaps; appended to `list`
 // starting at *count.  entry = block | extra | (in set 0) << 24 | (in set 1) << 25.
@@ -210,7 +233,7 @@ template <bool BF16, int D>
 __global__ void __launch_bounds__(kDkdvThreads, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tmap4 tmK,
                       const __grid_constant__ Tmap4 tmV, const __grid_constant__ Tmap4 tmDO,
-                      bsa_bwd_params bp, int* wait_status) {
+                      bsa_bwd_params bp, TileOrder order, int* wait_status) {
   const bsa_fwd_params& p = bp.f;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -230,8 +253,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // Long tiles first: adjacent pairs are longest at the low (causal) end already, the caller's
   // pairing table lists the pairs by ascending column length.
-  const int c2 = bp.kv_pairs ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-  const int hk = blockIdx.y, b = blockIdx.z;
+  int c2, hb;
+  tile_of_cta(order, &c2, &hb);
+  if (bp.kv_pairs) c2 = order.n_ranks - 1 - c2;
+  const int hk = hb % p.hkv, b = hb / p.hkv;
   const int G = p.hq / p.hkv;
   const int past = p.causal ? p.sk - p.sq : 0;
   // the two kv blocks of this tile: adjacent ones, or the caller's pairing
@@ -675,7 +700,7 @@ template <bool BF16, int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_sm100_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tmap4 tmK,
                     const __grid_constant__ Tmap4 tmV, const __grid_constant__ Tmap4 tmDO,
-                    bsa_bwd_params bp, int mode, int* wait_status) {
+                    bsa_bwd_params bp, int mode, TileOrder order, int* wait_status) {
   const bsa_fwd_params& p = bp.f;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -694,20 +719,23 @@ bwd_dq_sm100_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ T
   if (*reinterpret_cast<volatile int*>(wait_status) != 0) { wait_for_dkdv(); return; }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.hq / p.hkv;
-  const int b = blockIdx.z;
-  const int tile = gridDim.x - 1 - blockIdx.x;
+  int rank, hb;
+  tile_of_cta(order, &rank, &hb);
+  const int head_items = mode == kPairHeads ? p.hq / 2 : p.hq;
+  const int hy = hb % head_items, b = hb / head_items;
+  const int tile = order.n_ranks - 1 - rank;
   const int past = p.causal ? p.sk - p.sq : 0;
   int head[2], qblk[2], valid[2], kvh;
   if (mode == kPairHeads) {
     const int pairs = G / 2;
-    kvh = blockIdx.y / pairs;
-    head[0] = kvh * G + 2 * (blockIdx.y % pairs);
+    kvh = hy / pairs;
+    head[0] = kvh * G + 2 * (hy % pairs);
     head[1] = head[0] + 1;
     qblk[0] = qblk[1] = tile;
     valid[0] = valid[1] = 1;
   } else {
-    head[0] = head[1] = blockIdx.y;
-    kvh = blockIdx.y / G;
+    head[0] = head[1] = hy;
+    kvh = hy / G;
     qblk[0] = 2 * tile;
     qblk[1] = 2 * tile + 1;
     valid[0] = 1;
@@ -1043,7 +1071,8 @@ template <int D> constexpr size_t dqs_smem() {
 
 template <bool BF16, int D>
 __global__ void __launch_bounds__(kDqsThreads, 2)
-bwd_dq_from_ds_kernel(const __grid_constant__ Tmap4 tmK, bsa_bwd_params bp, int mode, int* wait_status) {
+bwd_dq_from_ds_kernel(const __grid_constant__ Tmap4 tmK, bsa_bwd_params bp, int mode, TileOrder order,
+                      int* wait_status) {
   const bsa_fwd_params& p = bp.f;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -1057,20 +1086,23 @@ bwd_dq_from_ds_kernel(const __grid_constant__ Tmap4 tmK, bsa_bwd_params bp, int 
   if (*reinterpret_cast<volatile int*>(wait_status) != 0) { wait_for_dkdv(); return; }
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.hq / p.hkv;
-  const int b = blockIdx.z;
-  const int tile = gridDim.x - 1 - blockIdx.x;
+  int rank, hb;
+  tile_of_cta(order, &rank, &hb);
+  const int head_items = mode == kPairHeads ? p.hq / 2 : p.hq;
+  const int hy = hb % head_items, b = hb / head_items;
+  const int tile = order.n_ranks - 1 - rank;
   const int past = p.causal ? p.sk - p.sq : 0;
   int head[2], qblk[2], valid[2], kvh;
   if (mode == kPairHeads) {
     const int pairs = G / 2;
-    kvh = blockIdx.y / pairs;
-    head[0] = kvh * G + 2 * (blockIdx.y % pairs);
+    kvh = hy / pairs;
+    head[0] = kvh * G + 2 * (hy % pairs);
     head[1] = head[0] + 1;
     qblk[0] = qblk[1] = tile;
     valid[0] = valid[1] = 1;
   } else {
-    head[0] = head[1] = blockIdx.y;
-    kvh = blockIdx.y / G;
+    head[0] = head[1] = hy;
+    kvh = hy / G;
     qblk[0] = 2 * tile;
     qblk[1] = 2 * tile + 1;
     valid[0] = 1;
@@ -1266,22 +1298,23 @@ int launch_bwd(const bsa_bwd_params* bp, cudaStream_t s) {
   {
     auto kern = bwd_dkdv_sm100_kernel<BF16, D>;
     BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDkdvSmem));
-    dim3 grid(bp->kv_pairs ? bp->n_pairs : cdiv_i(cdiv_i(p->sk, kBS), 2), p->hkv, p->batch);
-    kern<<<grid, kDkdvThreads, kDkdvSmem, s>>>(tmQ, tmK, tmV, tmDO, *bp, status);
+    const TileOrder order = tile_order(bp->kv_pairs ? bp->n_pairs : cdiv_i(cdiv_i(p->sk, kBS), 2), p->hkv * p->batch, 1);
+    kern<<<order.n_ranks * order.n_heads, kDkdvThreads, kDkdvSmem, s>>>(tmQ, tmK, tmV, tmDO, *bp, order, status);
     rc = check_launch("bwd_dkdv_sm100_kernel");
     if (rc) return rc;
   }
   const int G = p->hq / p->hkv;
   // as in the forward: two q heads share a tile only when they share a block list
   const int mode = (G % 2 == 0 && p->h_pat != p->hq) ? kPairHeads : kPairRows;
+  const TileOrder order = tile_order(cdiv_i(p->sq, mode == kPairHeads ? 64 : 128),
+                                     (mode == kPairHeads ? p->hq / 2 : p->hq) * p->batch, bp->ds_ws ? 2 : 1);
   if (bp->ds_ws) {
     // dQ from the dS tiles the dK/dV kernel has stored (one product per block)
     constexpr size_t kDqsSmem = dqs_smem<D>();
     auto kern = bwd_dq_from_ds_kernel<BF16, D>;
     BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqsSmem));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cdiv_i(p->sq, mode == kPairHeads ? 64 : 128), mode == kPairHeads ? p->hq / 2 : p->hq,
-                       p->batch);
+    cfg.gridDim = dim3(order.n_ranks * order.n_heads);
     cfg.blockDim = dim3(kDqsThreads);
     cfg.dynamicSmemBytes = kDqsSmem;
     cfg.stream = s;
@@ -1290,16 +1323,14 @@ int launch_bwd(const bsa_bwd_params* bp, cudaStream_t s) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmK, *bp, mode, status));
+    BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmK, *bp, mode, order, status));
     rc = check_launch("bwd_dq_from_ds_kernel");
   } else {
     auto kern = bwd_dq_sm100_kernel<BF16, D>;
     BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqSmem));
-    dim3 grid(cdiv_i(p->sq, mode == kPairHeads ? 64 : 128), mode == kPairHeads ? p->hq / 2 : p->hq,
-              p->batch);
     // programmatic dependent of the dK/dV kernel (see the kernels' first lines)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
+    cfg.gridDim = dim3(order.n_ranks * order.n_heads);
     cfg.blockDim = dim3(kBwdThreads);
     cfg.dynamicSmemBytes = kDqSmem;
     cfg.stream = s;
@@ -1308,7 +1339,7 @@ int launch_bwd(const bsa_bwd_params* bp, cudaStream_t s) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmQ, tmK, tmV, tmDO, *bp, mode, status));
+    BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmQ, tmK, tmV, tmDO, *bp, mode, order, status));
     rc = check_launch("bwd_dq_sm100_kernel");
   }
   return rc;
