@@ -1,8 +1,8 @@
 // Bandwidth-bound decode: one query token per sequence against contiguous K/V.
 //
 // Grid = (split, kv head x head group, sequence).  A CTA owns up to
-// blocks_per_split attended blocks of one (sequence, kv head): a producer warp
-// streams their K and V tiles (TMA boxes of kTok tokens x D) through a 64 KB
+// blocks_per_split attended blocks of one (sequence, kv head): one warp lists them, and
+// their K and V tiles (TMA boxes of kTok tokens x D) stream through a 64 KB
 // shared-memory ring (three CTAs fit per SM, so one CTA's prologue and epilogue
 // are covered by the loads of the other two).  Every tile pair ("unit") belongs to ONE of the
 // four consumer warps, so four units are worked on at a time and the fixed costs of a unit
@@ -126,15 +126,15 @@ template <int D, bool FP8> struct DecGeo {
 template <int D, bool FP8, int NT> struct DecodeSmem {
   // after the 1024-aligned ring
   alignas(16) uint16_t q[NT * 8][D];           // q heads of the group, zero rows behind them
-  uint64_t full[DecGeo<D, FP8>::kStages];
-  uint64_t empty[DecGeo<D, FP8>::kStages];
+  uint64_t k_full[DecGeo<D, FP8>::kStages];
+  uint64_t v_full[DecGeo<D, FP8>::kStages];
   float wm[kConsumers][NT * 8];
   float wl[kConsumers][NT * 8];
   int n_units;                                 // units of this CTA
-  int unit_pos[1];                             // first position of each unit: max_units entries
+  int2 unit[1];                                // first position of each unit and its place in the cache: max_units entries
 };
 template <int D, bool FP8, int NT> size_t dec_smem(int max_units) {
-  return 1024 + kRingBytes + sizeof(DecodeSmem<D, FP8, NT>) + sizeof(int) * (size_t)max_units;
+  return 1024 + kRingBytes + sizeof(DecodeSmem<D, FP8, NT>) + sizeof(int2) * (size_t)max_units;
 }
 
 // four e4m3 bytes of a word -> two f16x2: (byte 0, byte 1) and (byte 2, byte 3); exact
@@ -151,11 +151,11 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
 
 // NT: 8-column tiles of q heads (heads_per_cta <= 8 NT).
 //
-// Bound by HBM with a 16-bit cache; with an 8-bit cache by the latency of the consumer warps and the
-// fixed cost of a CTA (row lookup, first tile, merge of the warps: 6 us).  64 sequences of 1024..8192
-// tokens, 32/8 heads, D 128, local 16 + stride 8: 63 us for the 401 MB of a bf16 cache (6.3 TB/s), 48 us
-// for the 203 MB of an e4m3 cache; 71 and 72 us when all four warps shared a unit, 16 tokens each,
-// with the heads on the rows (per unit and warp 2000 cycles of arithmetic latency, four times over).
+// Bound by HBM with a 16-bit cache; with an 8-bit cache by the fixed cost of a CTA (row lookup, first
+// tiles, merge of the warps: 7 us) and the latency of a unit.  64 sequences of 1024..8192 tokens, 32/8
+// heads, D 128, local 16 + stride 8, with the merge kernel: 69 us for the 401 MB of a bf16 cache, 54 us for
+// the 203 MB of an e4m3 cache.  (78 and 79 us when all four warps shared a unit, 16 tokens each, with the
+// heads on the rows; 71 and 56 us when a producer warp refilled K and V together after both were read.)
 template <typename T, int D, bool FP8, int NT>
 __global__ void __launch_bounds__(kDecThreads, FP8 && D == 128 && NT == 2 ? 2 : kMinCtas)   // 2: spills otherwise
 decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 tmV,
@@ -174,7 +174,9 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
 
   // the merge kernel behind this one may be made resident as soon as every CTA got here
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (*reinterpret_cast<volatile int*>(wait_status) != 0) return;  // an earlier wait gave up
+  // non-zero: an earlier wait gave up.  Looked at after the row lookup, whose chain of dependent loads
+  // (ranges, row pointer, columns) is what a CTA begins with: no need to put this load in front of it.
+  const int gave_up = *reinterpret_cast<volatile int*>(wait_status);
   const int sp = blockIdx.x, b = blockIdx.z;
   // Row of q, o and lse: the sequence's number, or (packed batch of chunks and decode tokens) the
   // row of its single query token; sequences with another number of query tokens are not served here.
@@ -203,29 +205,25 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   // > 1, the blocks whose index is congruent to k_blk_rem modulo W, stored back to back (block c
   // of the sequence is local block c / W).
   const int mod = p.k_blk_mod > 1 ? p.k_blk_mod : 1;
-  auto issue_unit = [&](int u) {
+  auto load_tile = [&](int u, bool is_v) {
     const int s = u % kStages;
-    mbar_expect_tx(&sm->full[s], kStageBytes);
-    const int upos = sm->unit_pos[u];
-    const int tok = mod == 1 ? ks + (upos - pos0) : ks + (upos / bs / mod) * bs + upos % bs;
+    uint64_t* bar = is_v ? &sm->v_full[s] : &sm->k_full[s];
+    mbar_expect_tx(bar, kTileBytes);
+    const int tok = sm->unit[u].y;
     // a unit starts inside the stored tokens of its kv head (its tail may be past them)
     (void)BSA_IN_BOUNDS(tok >= 0 && tok < p.sk && kvh >= 0 && kvh < p.hkv && b < p.batch, wait_status, 821);
-    uint8_t* kdst = ring + s * kStageBytes;
-    uint8_t* vdst = kdst + kTileBytes;
-    if (FP8) {   // one box of [kTok tokens][D bytes] per tensor, as stored
-      tma_load_tile(kdst, &tmK, &sm->full[s], 0, tok, kvh, b);
-      tma_load_tile(vdst, &tmV, &sm->full[s], 0, tok, kvh, b);
-    } else {
+    uint8_t* dst = ring + s * kStageBytes + (is_v ? kTileBytes : 0);
+    const Tmap4* tm = is_v ? &tmV : &tmK;
+    // 8-bit: one box of [kTok tokens][D bytes], as stored
+    constexpr int kBoxes = FP8 ? 1 : D / 64;
 #pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
-        tma_load_tile(kdst + c * (kTok * 128), &tmK, &sm->full[s], c * 64, tok, kvh, b);
-        tma_load_tile(vdst + c * (kTok * 128), &tmV, &sm->full[s], c * 64, tok, kvh, b);
-      }
-    }
+    for (int c = 0; c < kBoxes; ++c) tma_load_tile(dst + c * (kTok * 128), tm, bar, c * 64, tok, kvh, b);
   };
 
   if (warp == kConsumers) {
-    // ---- the producer warp finds the attended blocks of this CTA: the sp-th group of
+    if (lane == 0) tma_prefetch_desc(&tmK.map);
+    if (lane == 1) tma_prefetch_desc(&tmV.map);
+    // ---- this warp finds the attended blocks of this CTA: the sp-th group of
     // blocks_per_split row entries that lie in the shard.  The row is read 32 entries at a time
     // (one coalesced load and one vote per chunk instead of a chain of dependent loads), and the
     // first tiles are requested before the rest of the CTA has staged Q.
@@ -256,7 +254,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
             const int pos = c * bs + s * kTok;
             const int u = (idx - want0) * subs + s;
             if (pos < end_pos && u < max_units) {
-              sm->unit_pos[u] = pos;
+              sm->unit[u] = make_int2(pos, mod == 1 ? ks + (pos - pos0) : ks + (c / mod) * bs + s * kTok);
               ++valid_units;
             }
           }
@@ -265,15 +263,17 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         seen += __popc(vote);
       }
     }
+    if (gave_up) nu = -1;
     __syncwarp();
     if (lane == 0) {
       sm->n_units = nu;
       for (int s = 0; s < kStages; ++s) {
-        mbar_init(&sm->full[s], 1);
-        mbar_init(&sm->empty[s], 1);   // the warp that owns the unit
+        mbar_init(&sm->k_full[s], 1);
+        mbar_init(&sm->v_full[s], 1);
       }
       mbar_fence_init();
-      for (int u = 0; u < nu && u < kStages; ++u) issue_unit(u);
+      for (int u = 0; u < nu && u < kStages; ++u) load_tile(u, false);
+      for (int u = 0; u < nu && u < kStages; ++u) load_tile(u, true);
     }
   } else {
     // q heads of the group -> rows of the q tile (rows >= GH are zero), 16 bytes a thread
@@ -303,6 +303,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   }
   __syncthreads();
   const int n_units = sm->n_units;
+  if (n_units < 0) return;   // outputs are undefined until the host has cleared the status
   // one split and an output tensor: write the final rows; otherwise an fp32 partial per split
   const bool final_out = nsplit == 1 && p.o != nullptr;
 
@@ -333,18 +334,10 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) oacc[i][nt][0] = oacc[i][nt][1] = oacc[i][nt][2] = oacc[i][nt][3] = 0.f;
 
-  if (warp == kConsumers) {
-    // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      for (int u = kStages; u < n_units; ++u) {   // the first kStages units are already in flight
-        const int s = u % kStages;
-        const uint32_t ph = (u / kStages) & 1;
-        if (!mbar_wait(&sm->empty[s], ph ^ 1, wait_status, 101)) break;
-        issue_unit(u);
-      }
-    }
-  } else {
+  if (warp < kConsumers) {
     // ------------------------------------------------------------ consumers
+    // A stage belongs to one warp, which asks for the next tile itself: K's place is refilled while the
+    // softmax and V^T P^T of the unit are computed, V's while the next unit's K Q^T is.
     uint32_t qb[D / 16][NT][2];   // Q^T as the B operand: column n = g is head 8 nt + g
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk)
@@ -369,23 +362,12 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     for (int u = warp; u < n_units; u += kConsumers) {
       const int s = u % kStages;
       const uint32_t ph = (u / kStages) & 1;
-      if (!mbar_wait(&sm->full[s], ph, wait_status, 102)) break;
+      if (!mbar_wait(&sm->k_full[s], ph, wait_status, 102)) break;
       const uint32_t kbase = ring_u32 + s * kStageBytes;
       const uint32_t vbase = kbase + kTileBytes;
       const uint8_t* k8 = ring + s * kStageBytes;    // the tiles as generic pointers (8-bit path)
       const uint8_t* v8 = k8 + kTileBytes;
-      const int valid = end_pos - sm->unit_pos[u];   // tokens of this unit that exist (may exceed kTok)
-      if (!FP8 && valid < kTok) {
-        // rows past the end of the sequence may hold anything: clear them in V so that 0 * garbage
-        // cannot produce NaN (the 8-bit path replaces them as it reads V)
-        uint8_t* vgen = ring + s * kStageBytes + kTileBytes;
-        for (int t = valid; t < kTok; ++t)
-#pragma unroll
-          for (int c = 0; c < D / 64; ++c)
-            reinterpret_cast<uint32_t*>(vgen + c * (kTok * 128) + t * 128)[lane] = 0u;
-        fence_proxy_async();  // order these writes before the next TMA into the stage
-        __syncwarp();
-      }
+      const int valid = end_pos - sm->unit[u].x;   // tokens of this unit that exist (may exceed kTok)
       // S^T = K Q^T
       float sacc[kTok / 16][NT][4];
 #pragma unroll
@@ -418,6 +400,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
           }
         }
       }
+      __syncwarp();   // every lane has read K
+      if (lane == 0 && u + kStages < n_units) load_tile(u + kStages, false);
       // mask; per head: maximum over the unit's tokens, reference maximum, sum
       float alpha[NT][2];
       bool need = false;
@@ -477,6 +461,18 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
           pb[mt][nt][1] = transpose8x8(MmaType<MT>::pack(p2, p3));
         }
       }
+      if (!mbar_wait(&sm->v_full[s], ph, wait_status, 101)) break;
+      if (!FP8 && valid < kTok) {
+        // rows past the end of the sequence may hold anything: clear them in V so that 0 * garbage
+        // cannot produce NaN (the 8-bit path replaces them as it reads V)
+        uint8_t* vgen = ring + s * kStageBytes + kTileBytes;
+        for (int t = valid; t < kTok; ++t)
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c)
+            reinterpret_cast<uint32_t*>(vgen + c * (kTok * 128) + t * 128)[lane] = 0u;
+        fence_proxy_async();  // order these writes before the next TMA into the stage
+        __syncwarp();
+      }
       // O^T += V^T P^T
 #pragma unroll
       for (int mt = 0; mt < kTok / 16; ++mt) {
@@ -519,8 +515,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
           }
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm->empty[s]);
+      __syncwarp();   // every lane has read V
+      if (lane == 0 && u + kStages < n_units) load_tile(u + kStages, true);
     }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
