@@ -180,10 +180,15 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   const int sp = blockIdx.x, b = blockIdx.z;
   // Row of q, o and lse: the sequence's number, or (packed batch of chunks and decode tokens) the
   // row of its single query token; sequences with another number of query tokens are not served here.
+  // That launch is a programmatic dependent of the prefill kernel, of which it reads nothing; no CTA
+  // leaves before that grid has completed, so that what follows in the stream follows both.
+  const auto leave = [&] {
+    if (row_start) asm volatile("griddepcontrol.wait;" ::: "memory");
+  };
   int qb = b;
   if (row_start) {
     qb = row_start[b];
-    if (row_end[b] - qb != 1) return;
+    if (row_end[b] - qb != 1) { leave(); return; }
   }
   const int G = p.hq / p.hkv;
   const int GH = p.heads_per_cta;
@@ -303,7 +308,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   }
   __syncthreads();
   const int n_units = sm->n_units;
-  if (n_units < 0) return;   // outputs are undefined until the host has cleared the status
+  if (n_units < 0) { leave(); return; }   // outputs are undefined until the host has cleared the status
   // one split and an output tensor: write the final rows; otherwise an fp32 partial per split
   const bool final_out = nsplit == 1 && p.o != nullptr;
 
@@ -324,6 +329,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         p.ws[(int64_t)p.batch * p.hq * nsplit * D + ((int64_t)b * p.hq + h) * nsplit + sp] = -INFINITY;
       }
     }
+    leave();
     return;
   }
 
@@ -592,6 +598,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         p.ws[(int64_t)p.batch * p.hq * nsplit * D + ((int64_t)b * p.hq + h) * nsplit + sp] = lse;
     }
   }
+  leave();
 }
 
 // out[row] = sum_p o_p[row] * softmax_p(lse_p[row]); merged lse = logsumexp_p.
@@ -712,7 +719,17 @@ int launch_decode(const bsa_decode_params* p, int nsplit, const int32_t* row_sta
   dim3 grid(nsplit, p->hkv * (G / p->heads_per_cta), p->batch);
   int* status = wait_status_ptr();
   if (!status) return BSA_E_CUDA;
-  kern<<<grid, kDecThreads, smem, s>>>(tmK, tmV, q, nsplit, max_units, row_start, row_end, status);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kDecThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = row_start ? 1 : 0;
+  BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, q, nsplit, max_units, row_start, row_end, status));
   rc = check_launch("decode_kernel");
   if (rc) return rc;
   if (nsplit > 1 && p->o) {

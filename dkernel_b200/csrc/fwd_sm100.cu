@@ -255,10 +255,10 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
   uint8_t* sRing = smem + kQBytes;      // slot s: K at s * 2 * kTile, V one kTile behind it
   TailP* tl = reinterpret_cast<TailP*>(smem + kQBytes + 2 * 2 * kTile);
 
-  if (*reinterpret_cast<volatile int*>(wait_status) != 0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    return;
-  }
+  // the single-token kernel behind this one reads nothing that this kernel writes: its CTAs may take
+  // the SMs that the last tiles leave idle
+  if (skip_single) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (*reinterpret_cast<volatile int*>(wait_status) != 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
@@ -686,9 +686,6 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
   tc_fence_before();
   __syncthreads();
   if (warp == kWarpIssue) tmem_dealloc(tmem, D <= 128 ? 256 : 512);
-  // Behind the single-token kernel (a programmatic dependent that reads nothing that kernel writes)
-  // no CTA leaves before that grid has completed, so that what follows in the stream follows both.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 }  // namespace
@@ -760,37 +757,11 @@ int launch_fwd(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStre
   constexpr size_t smem = Geo<D>::kSmem + sizeof(TailP);
   auto kern = fwd_persist_kernel<BF16, D, FB>;
   BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreadsP);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = skip_single ? 1 : 0;   // behind the single-token kernel, beside which it may run
-  BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmQ, tmK, tmV, *p, mode, n_items, tiles_x, head_items, zero_pads,
-                                    skip_single, status));
+  kern<<<grid, kThreadsP, smem, s>>>(tmQ, tmK, tmV, *p, mode, n_items, tiles_x, head_items, zero_pads, skip_single,
+                                     status);
   return check_launch("fwd_persist_kernel");
 }
-}  // namespace
-
-int sm100_fwd(const bsa_fwd_params* pp, cudaStream_t s) {
-  bsa_fwd_params q = *pp;
-  const bsa_fwd_params* p = &q;
-  const int zero_pads = q.row_mode == BSA_ROWS_BY_POSITION_ZERO_PADS;
-  if (zero_pads) q.row_mode = BSA_ROWS_BY_POSITION;
-  // A packed batch of prompt chunks and decode tokens (separate query ranges, which a prefill of whole
-  // prompts does not pass): sequences with one query token go to the decode kernel, which reads their
-  // K/V once for all heads of a group instead of walking them in 64-row tiles with one row in use.
-  // 3 chunks of 512 tokens and 45 decode tokens over 192 thousand keys, 32/8 heads, D 128: 197 -> 162 us.
-  const int skip_single = p->total_q > 0 && p->q_start != p->k_start && p->causal && p->fine_block == 0 &&
-                          p->row_mode == BSA_ROWS_BY_POSITION && (p->d == 64 || p->d == 128) && p->batch <= 65535;
-  if (skip_single) {
-    const int rc = decode_packed_rows(p, s);
-    if (rc) return rc;
-  }
+int launch_fwd_for(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStream_t s) {
   const bool bf16 = p->dtype == BSA_BF16;
   if (p->fine_block == 16) {
     if (p->d <= 64) return bf16 ? launch_fwd<true, 64, 16>(p, zero_pads, skip_single, s) : launch_fwd<false, 64, 16>(p, zero_pads, skip_single, s);
@@ -803,6 +774,23 @@ int sm100_fwd(const bsa_fwd_params* pp, cudaStream_t s) {
   if (p->d <= 64) return bf16 ? launch_fwd<true, 64, 0>(p, zero_pads, skip_single, s) : launch_fwd<false, 64, 0>(p, zero_pads, skip_single, s);
   if (p->d <= 128) return bf16 ? launch_fwd<true, 128, 0>(p, zero_pads, skip_single, s) : launch_fwd<false, 128, 0>(p, zero_pads, skip_single, s);
   return bf16 ? launch_fwd<true, 256, 0>(p, zero_pads, skip_single, s) : launch_fwd<false, 256, 0>(p, zero_pads, skip_single, s);
+}
+}  // namespace
+
+int sm100_fwd(const bsa_fwd_params* pp, cudaStream_t s) {
+  bsa_fwd_params q = *pp;
+  const bsa_fwd_params* p = &q;
+  const int zero_pads = q.row_mode == BSA_ROWS_BY_POSITION_ZERO_PADS;
+  if (zero_pads) q.row_mode = BSA_ROWS_BY_POSITION;
+  // A packed batch of prompt chunks and decode tokens (separate query ranges, which a prefill of whole
+  // prompts does not pass): sequences with one query token go to the decode kernel, which reads their
+  // K/V once for all heads of a group instead of walking them in 64-row tiles with one row in use.
+  // 3 chunks of 512 tokens and 45 decode tokens over 192 thousand keys, 32/8 heads, D 128: 197 us with
+  // all of them as tiles, 147 us with the decode kernel in front of this one, 135 us behind it.
+  const int skip_single = p->total_q > 0 && p->q_start != p->k_start && p->causal && p->fine_block == 0 &&
+                          p->row_mode == BSA_ROWS_BY_POSITION && (p->d == 64 || p->d == 128) && p->batch <= 65535;
+  const int rc = launch_fwd_for(p, zero_pads, skip_single, s);
+  return rc || !skip_single ? rc : decode_packed_rows(p, s);
 }
 
 }  // namespace bsa
