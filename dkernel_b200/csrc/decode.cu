@@ -37,6 +37,31 @@ constexpr int kMaxTokens = 4096;         // tokens per CTA (a caller's blocks_pe
 constexpr int kMaxRowBlocks = 1024;      // blocks of one row in a packed batch (decode_packed_rows)
 constexpr float kDecRescale = 8.0f;      // log2 of how far a maximum may grow before O is rescaled
 
+constexpr int kClusterCtas = 128;        // CTAs per resident CTA of an SM up to which a grid runs as clusters
+constexpr int kMaxCluster = 8;           // splits of a row that merge over distributed shared memory
+
+// every thread of the cluster's CTAs; what was written to shared memory before is visible behind it
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// reads of another CTA's shared memory: the address that `p` has there
+__device__ __forceinline__ uint32_t peer_smem(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float peer_load(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 peer_load4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+
 template <typename T> struct MmaType;
 template <> struct MmaType<__half> {
   static __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
@@ -159,7 +184,7 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
 template <typename T, int D, bool FP8, int NT>
 __global__ void __launch_bounds__(kDecThreads, FP8 && D == 128 && NT == 2 ? 2 : kMinCtas)   // 2: spills otherwise
 decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 tmV,
-              bsa_decode_params p, int nsplit, int max_units, const int32_t* __restrict__ row_start,
+              bsa_decode_params p, int nsplit, int cl, int max_units, const int32_t* __restrict__ row_start,
               const int32_t* __restrict__ row_end, int* wait_status) {
   using Geo = DecGeo<D, FP8>;
   constexpr int kStages = Geo::kStages, kTok = Geo::kTok;
@@ -244,7 +269,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       }
       const int32_t* cols = p.col + (int64_t)hp * p.col_sh;
       const int subs = bs / kTok;
-      const int want0 = sp * p.blocks_per_split, want1 = want0 + p.blocks_per_split;
+      // a cluster's CTAs take the entries in turns, which keeps their shares of any row level
+      const int want0 = cl > 1 ? 0 : sp * p.blocks_per_split, want1 = want0 + cl * p.blocks_per_split;
       int seen = 0;   // row entries of the shard met so far
       for (int e0 = c_beg; e0 < c_end && seen < want1; e0 += 32) {
         const int e = e0 + lane;
@@ -253,11 +279,11 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         const uint32_t vote = __ballot_sync(0xffffffffu, mine);
         const int idx = seen + __popc(vote & ((1u << lane) - 1u));
         int valid_units = 0;
-        if (mine && idx >= want0 && idx < want1) {
+        if (mine && idx >= want0 && idx < want1 && (cl == 1 || idx % cl == sp)) {
           for (int s = 0; s < subs; ++s) {
             // positions grow with the entry index, so the units past the end form a tail
             const int pos = c * bs + s * kTok;
-            const int u = (idx - want0) * subs + s;
+            const int u = (idx - want0) / cl * subs + s;
             if (pos < end_pos && u < max_units) {
               sm->unit[u] = make_int2(pos, mod == 1 ? ks + (pos - pos0) : ks + (c / mod) * bs + s * kTok);
               ++valid_units;
@@ -268,7 +294,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         seen += __popc(vote);
       }
     }
-    if (gave_up) nu = -1;
+    if (gave_up) nu = cl > 1 ? 0 : -1;   // no CTA of a cluster leaves before the others have read its part
     __syncwarp();
     if (lane == 0) {
       sm->n_units = nu;
@@ -312,7 +338,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   // one split and an output tensor: write the final rows; otherwise an fp32 partial per split
   const bool final_out = nsplit == 1 && p.o != nullptr;
 
-  if (n_units == 0) {  // nothing attended here: an empty partial (uniform exit)
+  if (n_units == 0 && cl == 1) {  // nothing attended here: an empty partial (uniform exit)
     for (int i = tid; i < GH * D; i += kDecThreads) {
       const int h = h0 + i / D, d = i % D;
       if (final_out) {
@@ -560,21 +586,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
 
   const bool o_vec = reinterpret_cast<uintptr_t>(p.o) % 8 == 0 && p.o_sb % 4 == 0 && p.o_sh % 4 == 0;
   const bool ws_vec = reinterpret_cast<uintptr_t>(p.ws) % 16 == 0;
-  for (int i = tid; i < GH * (D / 4); i += kDecThreads) {
-    const int r = i / (D / 4), d = i % (D / 4) * 4;
-    float mf = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kConsumers; ++w) mf = fmaxf(mf, sm->wm[w][r]);
-    const float msafe = mf == -INFINITY ? 0.f : mf;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float l = 0.f;
-#pragma unroll
-    for (int w = 0; w < kConsumers; ++w) {
-      const float sc = exp2f(sm->wm[w][r] - msafe);
-      const float4 v = *reinterpret_cast<const float4*>(Om + (w * NT * 8 + r) * kRow + d);
-      acc.x += v.x * sc; acc.y += v.y * sc; acc.z += v.z * sc; acc.w += v.w * sc;
-      l += sm->wl[w][r] * sc;
-    }
+  auto store = [&](int r, int d, float4 acc, float mf, float l) {
     const float inv = (l > 0.f ? 1.f / l : 0.f) * (FP8 ? p.v_scale : 1.f);   // e4m3 V: per-tensor scale
     const float lse = l > 0.f ? (mf + log2f(l)) * kLn2 : -INFINITY;
     acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
@@ -597,6 +609,60 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       if (d == 0)
         p.ws[(int64_t)p.batch * p.hq * nsplit * D + ((int64_t)b * p.hq + h) * nsplit + sp] = lse;
     }
+  };
+  // this CTA's part of a cluster's row: sums relative to the CTA's own maximum, behind the warps' parts
+  float* part = Om + kConsumers * NT * 8 * kRow;   // [NT * 8][D], then the maxima and the sums
+  float* part_m = part + NT * 8 * D;
+  float* part_l = part_m + NT * 8;
+  static_assert((kConsumers * NT * 8 * kRow + NT * 8 * (D + 2)) * 4 <= kRingBytes, "both must fit the ring");
+  for (int i = tid; i < GH * (D / 4); i += kDecThreads) {
+    const int r = i / (D / 4), d = i % (D / 4) * 4;
+    float mf = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kConsumers; ++w) mf = fmaxf(mf, sm->wm[w][r]);
+    const float msafe = mf == -INFINITY ? 0.f : mf;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+#pragma unroll
+    for (int w = 0; w < kConsumers; ++w) {
+      const float sc = exp2f(sm->wm[w][r] - msafe);
+      const float4 v = *reinterpret_cast<const float4*>(Om + (w * NT * 8 + r) * kRow + d);
+      acc.x += v.x * sc; acc.y += v.y * sc; acc.z += v.z * sc; acc.w += v.w * sc;
+      l += sm->wl[w][r] * sc;
+    }
+    if (cl == 1) {
+      store(r, d, acc, mf, l);
+    } else {
+      *reinterpret_cast<float4*>(part + r * D + d) = acc;
+      if (d == 0) { part_m[r] = mf; part_l[r] = l; }
+    }
+  }
+  if (cl > 1) {
+    cluster_sync();
+    // the CTAs share the rows' columns out among themselves
+    for (int i = tid * cl + sp; i < GH * (D / 4); i += kDecThreads * cl) {
+      const int r = i / (D / 4), d = i % (D / 4) * 4;
+      float mj[kMaxCluster];
+      float mf = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < kMaxCluster; ++j) {
+        mj[j] = j < cl ? peer_load(peer_smem(part_m + r, j)) : -INFINITY;
+        mf = fmaxf(mf, mj[j]);
+      }
+      const float msafe = mf == -INFINITY ? 0.f : mf;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      float l = 0.f;
+#pragma unroll
+      for (int j = 0; j < kMaxCluster; ++j) {
+        if (j >= cl) break;
+        const float sc = exp2f(mj[j] - msafe);
+        const float4 v = peer_load4(peer_smem(part + r * D + d, j));
+        acc.x += v.x * sc; acc.y += v.y * sc; acc.z += v.z * sc; acc.w += v.w * sc;
+        l += peer_load(peer_smem(part_l + r, j)) * sc;
+      }
+      store(r, d, acc, mf, l);
+    }
+    cluster_sync();   // the others have read this CTA's part
   }
   leave();
 }
@@ -694,7 +760,7 @@ int decode_nsplit(const bsa_decode_params* p) {
 }
 
 template <typename T, int D, bool FP8, int NT>
-int launch_decode(const bsa_decode_params* p, int nsplit, const int32_t* row_start, const int32_t* row_end,
+int launch_decode(const bsa_decode_params* p, int nsplit, int cl, const int32_t* row_start, const int32_t* row_end,
                   cudaStream_t s) {
   Tmap4 tmK, tmV;
   const bool bf16 = p->dtype == BSA_BF16;
@@ -716,7 +782,7 @@ int launch_decode(const bsa_decode_params* p, int nsplit, const int32_t* row_sta
   BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)dec_smem<D, FP8, NT>(kMaxRowBlocks * 64 / Geo::kTok)));
   const int G = p->hq / p->hkv;
-  dim3 grid(nsplit, p->hkv * (G / p->heads_per_cta), p->batch);
+  dim3 grid(cl > 1 ? cl : nsplit, p->hkv * (G / p->heads_per_cta), p->batch);
   int* status = wait_status_ptr();
   if (!status) return BSA_E_CUDA;
   cudaLaunchConfig_t cfg = {};
@@ -724,40 +790,40 @@ int launch_decode(const bsa_decode_params* p, int nsplit, const int32_t* row_sta
   cfg.blockDim = dim3(kDecThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = row_start ? 1 : 0;
-  BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, q, nsplit, max_units, row_start, row_end, status));
+  if (cl > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim = {(unsigned)cl, 1, 1};
+    ++cfg.numAttrs;
+  }
+  if (row_start) {   // behind the prefill kernel of the call
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  BSA_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, q, nsplit, cl, max_units, row_start, row_end, status));
   rc = check_launch("decode_kernel");
   if (rc) return rc;
   if (nsplit > 1 && p->o) {
     const int64_t rows = (int64_t)p->batch * p->hq;
     float* ws_lse = p->ws + rows * nsplit * D;
-    // partial o: (rows, nsplit, D) -> partition stride D, row stride nsplit*D
-    // the merged rows are written through (o_sb, o_sh): one launch per batch row
-    // layout unless o is contiguous over (batch, head)
-    // rows of o and lse may be strided (e.g. packed side by side in one buffer), but batch
-    // and head must collapse into one row index
-    if (p->o_sb == (int64_t)p->hq * p->o_sh && (!p->lse || p->lse_sb == (int64_t)p->hq * p->lse_sh)) {
-      if (bf16)
-        return launch_merge<float, __nv_bfloat16>(p->ws, ws_lse, nsplit, rows, D, D,
-                                                  (int64_t)nsplit * D, 1, nsplit, p->o, p->o_sh,
-                                                  p->lse, s, p->lse_sh);
-      return launch_merge<float, __half>(p->ws, ws_lse, nsplit, rows, D, D, (int64_t)nsplit * D, 1,
-                                         nsplit, p->o, p->o_sh, p->lse, s, p->lse_sh);
-    }
-    set_error("bsa_decode: with several splits o and lse need batch stride = heads x head stride");
-    return BSA_E_UNSUPPORTED;
+    // partial o: (rows, nsplit, D) -> partition stride D, row stride nsplit*D; rows of o and lse may be
+    // strided (e.g. packed side by side in one buffer), batch and head collapse into one row index
+    // (decode_run has checked that they do)
+    if (bf16)
+      return launch_merge<float, __nv_bfloat16>(p->ws, ws_lse, nsplit, rows, D, D, (int64_t)nsplit * D, 1, nsplit,
+                                                p->o, p->o_sh, p->lse, s, p->lse_sh);
+    return launch_merge<float, __half>(p->ws, ws_lse, nsplit, rows, D, D, (int64_t)nsplit * D, 1, nsplit, p->o,
+                                       p->o_sh, p->lse, s, p->lse_sh);
   }
   return BSA_OK;
 }
 
 template <typename T>
-int launch_decode_t(const bsa_decode_params* p, bool fp8, int nsplit, const int32_t* row_start,
+int launch_decode_t(const bsa_decode_params* p, bool fp8, int nsplit, int cl, const int32_t* row_start,
                     const int32_t* row_end, cudaStream_t s) {
-  auto go = [&](auto kernel) { return kernel(p, nsplit, row_start, row_end, s); };
+  auto go = [&](auto kernel) { return kernel(p, nsplit, cl, row_start, row_end, s); };
   if (p->heads_per_cta > 8) {
     if (fp8) return p->d == 128 ? go(launch_decode<T, 128, true, 2>) : go(launch_decode<T, 64, true, 2>);
     return p->d == 128 ? go(launch_decode<T, 128, false, 2>) : go(launch_decode<T, 64, false, 2>);
@@ -803,12 +869,26 @@ int decode_run(const bsa_decode_params* p, cudaStream_t s) {
   }
   const int nsplit = decode_nsplit(p);
   BSA_CHECK_ARG((nsplit == 1 && p->o) || p->ws, "bsa_decode: workspace required for %d splits", nsplit);
-  if (p->dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(p, fp8, nsplit, nullptr, nullptr, s);
-  return launch_decode_t<__half>(p, fp8, nsplit, nullptr, nullptr, s);
+  if (nsplit > 1 && p->o &&
+      (p->o_sb != (int64_t)p->hq * p->o_sh || (p->lse && p->lse_sb != (int64_t)p->hq * p->lse_sh))) {
+    set_error("bsa_decode: with several splits o and lse need batch stride = heads x head stride");
+    return BSA_E_UNSUPPORTED;
+  }
+  // Where the whole grid is resident at once with some room to spare, up to eight splits are a cluster whose
+  // CTAs merge their parts over distributed shared memory: no partials and no second launch.  In a larger
+  // grid waiting for a cluster's worth of room costs more than the second launch.  (Sequences of 3000 to 4096
+  // tokens, 32/8 heads, D 128, 64 CTAs each: 1: 13.3 -> 11.3 us, 2: 13.3 -> 11.9, 4: 14.0 -> 13.3, 6: 15.4 ->
+  // 13.3, 8: 17.1 -> 21.5 us; 64 of 1024 to 8192 tokens: 69 -> 71 us.)
+  const long long ctas = (long long)p->batch * (p->hq / p->heads_per_cta) * nsplit;
+  const int resident = fp8 && p->d == 128 && p->heads_per_cta > 8 ? 2 : kMinCtas;   // the kernel's launch bounds
+  const int cl = p->o && nsplit > 1 && nsplit <= kMaxCluster && ctas <= kClusterCtas * resident ? nsplit : 1;
+  if (p->dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(p, fp8, cl > 1 ? 1 : nsplit, cl, nullptr, nullptr, s);
+  return launch_decode_t<__half>(p, fp8, cl > 1 ? 1 : nsplit, cl, nullptr, nullptr, s);
 }
 
 // The sequences of a packed batch that have one query token.  A CTA walks a whole pattern row (there
-// is no scratch for partials); its list holds every block of the pattern's longest possible row.
+// is no scratch for partials); its list holds every block of the pattern's longest possible row.  (Two or
+// four CTAs per row as a cluster: 163 and 221 us for the batch of sm100_fwd's comment, against 135.)
 int decode_packed_rows(const bsa_fwd_params* f, cudaStream_t s) {
   if (f->n_rows > kMaxRowBlocks && f->sk > kMaxRowBlocks * 64) {
     set_error("bsa_fwd: a row of a packed batch has more than %d blocks", kMaxRowBlocks);
@@ -832,11 +912,12 @@ int decode_packed_rows(const bsa_fwd_params* f, cudaStream_t s) {
     for (int c = 2; c <= G && c <= 16; ++c)
       if (G % c == 0) p.heads_per_cta = c;
   // columns ascend and a causal row sees no block past the sequence: its first cdiv(sk, 64) entries do
-  p.blocks_per_split = p.max_row_nnz = f->n_rows < cdiv_i(f->sk, 64) ? f->n_rows : cdiv_i(f->sk, 64);
+  p.max_row_nnz = f->n_rows < cdiv_i(f->sk, 64) ? f->n_rows : cdiv_i(f->sk, 64);
+  p.blocks_per_split = p.max_row_nnz;
   p.dtype = f->dtype;
   p.sm_scale = f->sm_scale;
-  if (p.dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(&p, false, 1, f->q_start, f->q_end, s);
-  return launch_decode_t<__half>(&p, false, 1, f->q_start, f->q_end, s);
+  if (p.dtype == BSA_BF16) return launch_decode_t<__nv_bfloat16>(&p, false, 1, 1, f->q_start, f->q_end, s);
+  return launch_decode_t<__half>(&p, false, 1, 1, f->q_start, f->q_end, s);
 }
 
 int merge_partials(const void* o_parts, const float* lse_parts, int P, int64_t rows, int d,

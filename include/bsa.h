@@ -219,8 +219,9 @@ int bsa_bwd(const bsa_bwd_params* p, void* stream);
  * Replaces the q_len == 1 launches of _fwd_kernel_batch_inference
  * (dkernel/ops/sparse_attn_inference.py:83-88, :141) and the sliced-crow decode
  * of _forward (dkernel/ops/sparse_attn_fwd.py:435-440).  Split-KV: every
- * (sequence, kv head, split) is one CTA; partial (O, m, l) go to the workspace
- * and are merged by a second kernel.
+ * (sequence, kv head, split) is one CTA; the partial (O, m, l) of small grids are
+ * merged inside the launch, others go to the workspace and are merged by a second
+ * kernel.
  * ------------------------------------------------------------------------- */
 typedef struct {
   const void* q;              /* (batch, hq, d), strides q_sb, q_sh             */

@@ -487,3 +487,26 @@ def test_packed_single_token_sequences_beside_chunks(Hq, Hkv, D, dtype, user_pat
         out, lse = mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda(), return_lse=True)
     assert_out_close(out, ref)
     assert_lse_close(lse, ref_lse)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,D,bps", [(4, 1, 128, 9), (4, 1, 128, 4), (8, 8, 64, 3), (16, 1, 128, 2), (4, 2, 128, 1)])
+def test_decode_split_counts(fp8, Hq, Hkv, D, bps):
+    """Two to eight splits of a row are merged inside a cluster, more (the last case) by a second launch; rows
+    with fewer blocks than splits leave some CTAs without work."""
+    from dkernel_b200.ops import decode
+    bs, lens = 64, [1, 64, 65, 200, 640, 1024, 1000]
+    B, S = len(lens), 1024
+    pk = dict(block_size=bs, local_blocks=16, vert_stride=4, num_kv_heads=Hkv)      # dense: up to 16 blocks a row
+    q, k, v = seeded_qkv(91, (B, 1, Hq, D), (B, S, Hkv, D), torch.bfloat16)
+    scales = (0.02, 0.015) if fp8 else None
+    if fp8:
+        k, v = (k.float() / scales[0]).to(torch.float8_e4m3fn), (v.float() / scales[1]).to(torch.float8_e4m3fn)
+    kf, vf = (k.float() * scales[0], v.float() * scales[1]) if fp8 else (k.float(), v.float())
+    left = torch.tensor([S - n for n in lens], dtype=torch.int32)
+    ref, ref_lse = O.decode_attention(q.float(), kf, vf, O.block_mask(Hq, S, **pk), bs, left_paddings=left)
+    mod = _module(Hq, S, pk, seq_dim=1)
+    out, lse = decode(q.cuda(), k.cuda(), v.cuda(), mod._plan(), 1.0 / math.sqrt(D), seq_dim=1, k_start=left.cuda(),
+                      blocks_per_split=bps, kv_scales=scales)
+    assert_out_close(out, ref)
+    assert_lse_close(lse.unsqueeze(-1), ref_lse)
