@@ -535,22 +535,41 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
             for (int c = 0; c < 64; ++c)
               if (c >= lim) sv[c] = 0xff800000u;  // -inf
           }
-          if (FB && cm != kFull) {
+          if (FB == 16 && cm != kFull) {
 #pragma unroll
             for (int c = 0; c < 64; ++c)
               if (!((cm >> (c / (FB ? FB : 1))) & 1u)) sv[c] = 0xff800000u;
           }
-          float m4[4];
+          // 32-token blocks: a warp's 32 rows are one sub-row, so all of them attend the same of the two
+          // 32-column halves and the other half costs neither a maximum nor exponentials (2 prompts of
+          // 4000 tokens, 16 heads, D 64, local 16 + stride 8: 75 -> 66 us)
+          if (FB == 32) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) m4[i] = max3(__uint_as_float(sv[3 * i]), __uint_as_float(sv[3 * i + 1]),
-                                                   __uint_as_float(sv[3 * i + 2]));
+            for (int hlf = 0; hlf < 2; ++hlf)
+              if ((cm >> hlf) & 1u) {
+                float m2[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-          for (int c = 12; c < 60; c += 8)
+                for (int c = 0; c < 32; c += 4)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              m4[i] = max3(m4[i], __uint_as_float(sv[c + 2 * i]), __uint_as_float(sv[c + 2 * i + 1]));
-          mx = max3(max3(m4[0], m4[1], m4[2]), max3(m4[3], __uint_as_float(sv[60]), __uint_as_float(sv[61])),
-                    fmaxf(__uint_as_float(sv[62]), __uint_as_float(sv[63]))) * scale2;
+                  for (int i = 0; i < 2; ++i)
+                    m2[i] = max3(m2[i], __uint_as_float(sv[hlf * 32 + c + 2 * i]),
+                                 __uint_as_float(sv[hlf * 32 + c + 2 * i + 1]));
+                mx = max3(mx, m2[0], m2[1]);
+              }
+            mx *= scale2;
+          } else {
+            float m4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) m4[i] = max3(__uint_as_float(sv[3 * i]), __uint_as_float(sv[3 * i + 1]),
+                                                     __uint_as_float(sv[3 * i + 2]));
+#pragma unroll
+            for (int c = 12; c < 60; c += 8)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                m4[i] = max3(m4[i], __uint_as_float(sv[c + 2 * i]), __uint_as_float(sv[c + 2 * i + 1]));
+            mx = max3(max3(m4[0], m4[1], m4[2]), max3(m4[3], __uint_as_float(sv[60]), __uint_as_float(sv[61])),
+                      fmaxf(__uint_as_float(sv[62]), __uint_as_float(sv[63]))) * scale2;
+          }
         }
         float alpha = 1.f;
         bool need = false;
@@ -576,7 +595,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
 #pragma unroll
         for (int hlf = 0; hlf < 2; ++hlf) {
           uint32_t pk[16];
-          if (live) {
+          if (live && (FB != 32 || ((cm >> hlf) & 1u))) {
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
               float x0, x1;
