@@ -219,9 +219,10 @@ __device__ __forceinline__ bool build_plan(const bsa_fwd_params& p, int mode, in
 
 // Padded batch: the rows of a tile behind the sequence's q_len stand for the storage rows outside
 // [q_start, q_start + q_len) (relative row r is storage row (q_start + r) mod sq, which covers all
-// of them once): zero rows, LSE = -inf.  `r0`: first of the warp's 32 rows.  Written here, the pads
-// cost neither a pass over the whole output before the kernel nor a launch, and hide behind the
-// arithmetic of the other warps (8 prompts of 256..2048 tokens padded to 2048, 32/8 heads, D 128:
+// of them once): zero rows, LSE = -inf.  Written here, the pads
+// cost neither a pass over the whole output before the kernel nor a launch; the planner warp, which
+// is idle most of the time, stores them (in the softmax warps the code alone, never run, cost packed
+// batches 1 %).  `r0`: first of 32 rows.  (8 prompts of 256..2048 tokens padded to 2048, 32/8 heads, D 128:
 // 213 us with the two fills, 182 us now, device time).
 __device__ __forceinline__ void store_pad_rows(const bsa_fwd_params& p, int head, int b, int q_start, int r0,
                                                int q_len, int lane, bool wide) {
@@ -317,6 +318,16 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
         break;
       }
       if (lane == 0) mbar_arrive(&tl->plan_full[pb]);
+      if (zero_pads) {
+        const Plan* pl = &tl->plan[pb];   // rewritten by this warp only
+        const bool wide = reinterpret_cast<uintptr_t>(p.o) % 16 == 0 && p.o_ss % 8 == 0 && p.o_sh % 8 == 0 &&
+                          p.o_sb % 8 == 0;
+        for (int i = 0; i < 4; ++i) {
+          const int r0 = pl->qblk[i >> 1] * kBS + (i & 1) * 32;
+          if (r0 + 32 > pl->q_len)
+            store_pad_rows(p, pl->head[i >> 1], pl->b, pl->q_start, r0, pl->q_len, lane, wide);
+        }
+      }
     }
   } else if (warp == kWarpProd) {
     // ============================================================ TMA producer
@@ -483,8 +494,6 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
                       ((int64_t)b * p.o_sb + (int64_t)head * p.o_sh + (int64_t)(pl->q_start + q_row) * p.o_ss) * 2;
       float* lse_ptr = p.lse ? p.lse + (int64_t)b * p.lse_sb + (int64_t)head * p.lse_sh + pl->q_start + q_row
                              : nullptr;
-      if (zero_pads && pl->qblk[t] * kBS + (warp & 1) * 32 + 32 > q_len)
-        store_pad_rows(p, head, b, pl->q_start, pl->qblk[t] * kBS + (warp & 1) * 32, q_len, lane, wide);
       if (n == 0) {
         if (pl->valid && row_ok) {   // a tile that attends nothing: zero rows, LSE = -inf
           for (int i = 0; i < p.d / 4; ++i) reinterpret_cast<uint2*>(orow)[i] = make_uint2(0u, 0u);
