@@ -223,6 +223,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int bs = p.block_size;
   const bool q_vec = reinterpret_cast<uintptr_t>(p.q) % 16 == 0 && p.q_sb % 8 == 0 && p.q_sh % 8 == 0;
+  // e4m3 K carries a per-tensor scale: it folds into the logit scale (V's goes on the output)
+  const float scale2 = p.sm_scale * kLog2e * (FP8 ? p.k_scale : 1.f);
 
   const int ks = p.k_start ? p.k_start[b] : 0;
   const int ke = p.k_end ? p.k_end[b] : p.sk;
@@ -307,7 +309,9 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       for (int u = 0; u < nu && u < kStages; ++u) load_tile(u, true);
     }
   } else {
-    // q heads of the group -> rows of the q tile (rows >= GH are zero), 16 bytes a thread
+    // q heads of the group -> rows of the q tile (rows >= GH are zero), 16 bytes a thread.  The maximum is
+    // taken and the end of the sequence masked before the logits are scaled, which asks for a positive
+    // scale: a negative one hands its sign to q here, and scale 0 makes the products themselves zero.
     for (int i = tid; i < NT * 8 * D / 8; i += kConsumers * 32) {
       const int r = i / (D / 8), c = i % (D / 8);
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -320,6 +324,11 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
 #pragma unroll
           for (int e = 0; e < 8; ++e) tmp[e] = src[e];
           v = *reinterpret_cast<const uint4*>(tmp);
+        }
+        if (!(scale2 > 0.f)) {
+          T* e = reinterpret_cast<T*>(&v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) e[j] = Elem<T>::from_f(Elem<T>::to_f(e[j]) * (scale2 < 0.f ? -1.f : scale2));
         }
         if (!std::is_same<MT, T>::value) {   // bf16 queries against an 8-bit cache: products run in f16
           const T* e = reinterpret_cast<const T*>(&v);
@@ -387,8 +396,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
     float m[NT][2], l[NT][2];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) { m[nt][0] = m[nt][1] = -INFINITY; l[nt][0] = l[nt][1] = 0.f; }
-    // e4m3 K carries a per-tensor scale: it folds into the logit scale (V's goes on the output)
-    const float scale2 = p.sm_scale * kLog2e * (FP8 ? p.k_scale : 1.f);
+    const float mul = scale2 == 0.f ? 1.f : fabsf(scale2);   // q carries the sign
     const uint32_t ring_u32 = smem_u32(ring);
 
     for (int u = warp; u < n_units; u += kConsumers) {
@@ -456,7 +464,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-          mx *= scale2;
+          mx *= mul;
           alpha[nt][e] = 1.f;
           if (m[nt][e] == -INFINITY) {
             m[nt][e] = mx;         // nothing summed so far
@@ -485,8 +493,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
         const float n0 = m[nt][0] == -INFINITY ? 0.f : -m[nt][0], n1 = m[nt][1] == -INFINITY ? 0.f : -m[nt][1];
 #pragma unroll
         for (int mt = 0; mt < kTok / 16; ++mt) {
-          const float p0 = dec_ex2(fmaf(sacc[mt][nt][0], scale2, n0)), p1 = dec_ex2(fmaf(sacc[mt][nt][1], scale2, n1));
-          const float p2 = dec_ex2(fmaf(sacc[mt][nt][2], scale2, n0)), p3 = dec_ex2(fmaf(sacc[mt][nt][3], scale2, n1));
+          const float p0 = dec_ex2(fmaf(sacc[mt][nt][0], mul, n0)), p1 = dec_ex2(fmaf(sacc[mt][nt][1], mul, n1));
+          const float p2 = dec_ex2(fmaf(sacc[mt][nt][2], mul, n0)), p3 = dec_ex2(fmaf(sacc[mt][nt][3], mul, n1));
           l[nt][0] += p0 + p2;
           l[nt][1] += p1 + p3;
           pb[mt][nt][0] = transpose8x8(MmaType<MT>::pack(p0, p1));

@@ -510,3 +510,53 @@ def test_decode_split_counts(fp8, Hq, Hkv, D, bps):
                       blocks_per_split=bps, kv_scales=scales)
     assert_out_close(out, ref)
     assert_lse_close(lse.unsqueeze(-1), ref_lse)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("scale", [-0.09, 0.0])
+@pytest.mark.parametrize("Hq,Hkv,D,dtype,bps", [
+    (4, 1, 128, torch.bfloat16, 0),     # splits merged inside a cluster
+    (4, 2, 64, torch.float16, 16),      # one split
+    (12, 1, 64, torch.bfloat16, 1),     # two column tiles, splits merged by a second launch
+])
+def test_decode_with_a_scale_that_is_not_positive(fp8, scale, Hq, Hkv, D, dtype, bps):
+    """The sign of the scale turns the order of the logits round, and scale 0 makes all of them equal: in full
+    units (the reference maximum) and in partial ones (the mask), on padded and packed caches.  Logits spread
+    over +-40, so that a reference taken from the wrong end overflows.  Bounds: the helpers' defaults."""
+    from dkernel_b200.ops import decode
+    bs, S, lens = 64, 1024, [1, 31, 33, 63, 64, 65, 200, 1000, 1024]
+    B = len(lens)
+    pk = dict(block_size=bs, local_blocks=16, vert_stride=4, num_kv_heads=Hkv)      # dense: up to 16 blocks a row
+    q, k, v = seeded_qkv(93, (B, 1, Hq, D), (B, S, Hkv, D), dtype)
+    q = q * 8
+    scales, kw = (0.02, 0.015), {}
+    if fp8:
+        k, v = (k.float() / scales[0]).to(torch.float8_e4m3fn), (v.float() / scales[1]).to(torch.float8_e4m3fn)
+        kw["kv_scales"] = scales
+    kf, vf = (k.float() * scales[0], v.float() * scales[1]) if fp8 else (k.float(), v.float())
+    left = torch.tensor([S - n for n in lens], dtype=torch.int32)
+    ref, ref_lse = O.decode_attention(q.float(), kf, vf, O.block_mask(Hq, S, **pk), bs, sm_scale=scale, left_paddings=left)
+    mod = _module(Hq, S, pk, seq_dim=1)
+    out, lse = decode(q.cuda(), k.cuda(), v.cuda(), mod._plan(), scale, seq_dim=1, k_start=left.cuda(),
+                      blocks_per_split=bps, **kw)
+    assert_out_close(out, ref)
+    assert_lse_close(lse.unsqueeze(-1), ref_lse)
+    cu = torch.tensor(np.cumsum([0] + lens), dtype=torch.int32).cuda()
+    kp, vp = (torch.cat([t[i, S - n:].view(torch.uint8) for i, n in enumerate(lens)]).view(t.dtype) for t in (k, v))
+    out, lse = decode(q[:, 0].cuda(), kp.cuda(), vp.cuda(), mod._plan(), scale, seq_dim=None, k_start=cu[:-1], k_end=cu[1:],
+                      blocks_per_split=bps, **kw)
+    assert_out_close(out, ref[:, 0])
+    assert_lse_close(lse.unsqueeze(-1), ref_lse)
+
+
+@pytest.mark.parametrize("n", [40, 64])
+def test_negative_scale_decode_is_the_last_row_of_the_prefill(n):
+    """One module, one scale: the token that a decode step computes is the last one of the prefill."""
+    pk = dict(block_size=64, local_blocks=2, vert_stride=3, num_kv_heads=2)
+    q, k, v = (t.cuda() for t in seeded_qkv(95, (1, n, 4, 64), (1, n, 2, 64), torch.float16))
+    mod = _module(4, 512, pk, seq_dim=1)
+    left = torch.zeros(1, dtype=torch.int32, device="cuda")
+    with torch.no_grad():
+        pre = mod(q, k, v, sm_scale=-0.2, left_paddings=left)
+        out = mod(q[:, -1:].contiguous(), k, v, sm_scale=-0.2, left_paddings=left)
+    assert_out_close(out, pre[:, -1:])
