@@ -62,6 +62,7 @@ struct TailP {
   // epilogue: 32 rows x 64 bytes per softmax warp, so that a store instruction covers whole
   // 64-byte row pieces of eight rows instead of 16 bytes of thirty-two rows
   alignas(16) uint8_t ostage[4][2048];
+  alignas(16) uint8_t zero_row[512];   // source of a padded batch's pad rows
 };
 
 
@@ -219,25 +220,26 @@ __device__ __forceinline__ bool build_plan(const bsa_fwd_params& p, int mode, in
 
 // Padded batch: the rows of a tile behind the sequence's q_len stand for the storage rows outside
 // [q_start, q_start + q_len) (relative row r is storage row (q_start + r) mod sq, which covers all
-// of them once): zero rows, LSE = -inf.  Written here, the pads
-// cost neither a pass over the whole output before the kernel nor a launch; the planner warp, which
-// is idle most of the time, stores them (in the softmax warps the code alone, never run, cost packed
-// batches 1 %).  `r0`: first of 32 rows.  (8 prompts of 256..2048 tokens padded to 2048, 32/8 heads, D 128:
-// 213 us with the two fills, 182 us now, device time).
+// of them once): zero rows, LSE = -inf.  `r0`: first of 32 rows, one per lane of the planner warp.
+// Written here, the pads cost neither a pass over the whole output before the kernel nor a launch.  A
+// row is one bulk copy of zeros from shared memory, so the warp is back at its plans at once.
+// (8 prompts of 256..2048 tokens padded to 2048, 32/8 heads, D 128: 224 us per call with the two fills
+// before the kernel, 221 with plain 16-byte stores by this warp, which kept it from planning, 202 now.
+// From the softmax warps: 203, but there the code alone, never run, costs packed batches 1 %.)
 __device__ __forceinline__ void store_pad_rows(const bsa_fwd_params& p, int head, int b, int q_start, int r0,
-                                               int q_len, int lane, bool wide) {
-  const int bytes = wide ? 16 : 8, pieces = p.d * 2 / bytes;
-  uint8_t* base = reinterpret_cast<uint8_t*>(p.o) + ((int64_t)b * p.o_sb + (int64_t)head * p.o_sh) * 2;
-  for (int i = lane; i < 32 * pieces; i += 32) {
-    const int r = r0 + i / pieces;
-    if (r < q_len || r >= p.sq) continue;
-    uint8_t* dst = base + (int64_t)((q_start + r) % p.sq) * p.o_ss * 2 + (i % pieces) * bytes;
-    if (wide) *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
-    else *reinterpret_cast<uint2*>(dst) = make_uint2(0u, 0u);
-  }
+                                               int q_len, int lane, bool wide, const void* zero_row, int* wait_status) {
   const int r = r0 + lane;
-  if (p.lse && r >= q_len && r < p.sq)
-    p.lse[(int64_t)b * p.lse_sb + (int64_t)head * p.lse_sh + (q_start + r) % p.sq] = -INFINITY;
+  if (r < q_len || r >= p.sq) return;
+  const int row = (q_start + r) % p.sq;
+  if (!BSA_IN_BOUNDS(row >= 0 && row < p.sq, wait_status, 807)) return;
+  uint8_t* dst = reinterpret_cast<uint8_t*>(p.o) +
+                 ((int64_t)b * p.o_sb + (int64_t)head * p.o_sh + (int64_t)row * p.o_ss) * 2;
+  if (wide) {   // 16-byte aligned; a row's bytes are a multiple of 16
+    bulk_store(dst, zero_row, p.d * 2);
+  } else {
+    for (int i = 0; i < p.d / 4; ++i) reinterpret_cast<uint2*>(dst)[i] = make_uint2(0u, 0u);
+  }
+  if (p.lse) p.lse[(int64_t)b * p.lse_sb + (int64_t)head * p.lse_sh + row] = -INFINITY;
 }
 
 // FB: 0, or the pattern's own block size (16 or 32) when it is finer than the 64-token tiles: the
@@ -296,6 +298,13 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
     // items from it as they go (long tiles first, so the CTAs finish within one short tile of
     // each other); without one, round r hands items [r * grid, (r + 1) * grid) to the CTAs,
     // odd rounds in reverse CTA order so that no CTA collects the longest tile of every round.
+    const bool wide = reinterpret_cast<uintptr_t>(p.o) % 16 == 0 && p.o_ss % 8 == 0 && p.o_sh % 8 == 0 &&
+                      p.o_sb % 8 == 0;
+    if (zero_pads) {
+      reinterpret_cast<uint4*>(tl->zero_row)[lane] = make_uint4(0u, 0u, 0u, 0u);
+      fence_proxy_async();   // generic-proxy writes -> visible to the bulk copies
+      __syncwarp();
+    }
     for (int k = 0;; ++k) {
       int item;
       if (p.tile_counter) {
@@ -320,15 +329,16 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
       if (lane == 0) mbar_arrive(&tl->plan_full[pb]);
       if (zero_pads) {
         const Plan* pl = &tl->plan[pb];   // rewritten by this warp only
-        const bool wide = reinterpret_cast<uintptr_t>(p.o) % 16 == 0 && p.o_ss % 8 == 0 && p.o_sh % 8 == 0 &&
-                          p.o_sb % 8 == 0;
         for (int i = 0; i < 4; ++i) {
           const int r0 = pl->qblk[i >> 1] * kBS + (i & 1) * 32;
           if (r0 + 32 > pl->q_len)
-            store_pad_rows(p, pl->head[i >> 1], pl->b, pl->q_start, r0, pl->q_len, lane, wide);
+            store_pad_rows(p, pl->head[i >> 1], pl->b, pl->q_start, r0, pl->q_len, lane, wide, tl->zero_row,
+                           wait_status);
         }
+        bulk_commit();
       }
     }
+    if (zero_pads) bulk_wait_all();   // the copies read shared memory
   } else if (warp == kWarpProd) {
     // ============================================================ TMA producer
     if (lane == 0) {

@@ -560,3 +560,29 @@ def test_negative_scale_decode_is_the_last_row_of_the_prefill(n):
         pre = mod(q, k, v, sm_scale=-0.2, left_paddings=left)
         out = mod(q[:, -1:].contiguous(), k, v, sm_scale=-0.2, left_paddings=left)
     assert_out_close(out, pre[:, -1:])
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,extra", [(4, 2, 128, 0), (2, 2, 72, 4), (4, 2, 256, 0), (2, 1, 16, 12)])
+def test_pad_rows_of_empty_sequences_and_of_unaligned_outputs(Hq, Hkv, D, extra):
+    """A sequence of nothing but pads, and pad rows of an output whose rows start 8 bytes off a 16-byte boundary
+    (``extra`` elements behind every row, which must keep what they hold).  The kernel's own real rows are the
+    reference's (an aligned output), the pad rows zero, LSE -inf."""
+    from dkernel_b200 import _lib, ops
+    B, S, bs = 4, 200, 64
+    pk = dict(block_size=bs, local_blocks=2, vert_stride=3, num_kv_heads=Hkv)
+    q, k, v = (t.cuda() for t in seeded_qkv(97, (B, S, Hq, D), (B, S, Hkv, D), torch.bfloat16))
+    left = torch.tensor([S, 0, S - 1, 77], dtype=torch.int32, device="cuda")
+    plan = _module(Hq, 256, pk, seq_dim=1)._plan()
+    buf = torch.full((B, S, Hq, D + extra), 7.0, dtype=q.dtype, device="cuda")
+    o, lse = buf[..., :D], torch.full((B, Hq, S), float("nan"), device="cuda")
+    ends = torch.full((B,), S, dtype=torch.int32, device="cuda")
+    p = ops._fwd_params(q, k, v, o, lse, 1, plan, 0.1, True, _lib.ROWS_BY_POSITION_ZERO_PADS, left, ends, left, ends,
+                        impl=_lib.IMPL_SM100)
+    ops._launch_fwd(p, q)
+    ref, ref_lse = O.padded_attention(q.float().cpu(), k.float().cpu(), v.float().cpu(), O.block_mask(Hq, 256, **pk), bs,
+                                      sm_scale=0.1, left_paddings=left.cpu())
+    assert_out_close(o, ref)
+    assert_lse_close(lse, ref_lse)
+    pad = torch.arange(S, device="cuda")[None] < left[:, None]
+    assert (o[pad] == 0).all() and torch.isneginf(lse.transpose(1, 2)[pad]).all()
+    assert (buf[..., D:] == 7.0).all()
