@@ -205,10 +205,12 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
   const int sp = blockIdx.x, b = blockIdx.z;
   // Row of q, o and lse: the sequence's number, or (packed batch of chunks and decode tokens) the
   // row of its single query token; sequences with another number of query tokens are not served here.
-  // That launch is a programmatic dependent of the prefill kernel, of which it reads nothing; no CTA
-  // leaves before that grid has completed, so that what follows in the stream follows both.
+  // That launch is a programmatic dependent of the prefill kernel, of which it reads nothing; its first
+  // CTA does not leave before that grid has completed, so that what follows in the stream follows both.
+  // The others leave when they are done: waiting, they would hold the places of rows still to be worked on
+  // (24 chunks of 64 tokens + 8 decode tokens: 106 -> 92 us; 7 chunks + 1 token: 43.7 -> 34 us).
   const auto leave = [&] {
-    if (row_start) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (row_start && blockIdx.x + blockIdx.y + blockIdx.z == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   };
   int qb = b;
   if (row_start) {

@@ -824,9 +824,14 @@ int sm100_fwd(const bsa_fwd_params* pp, cudaStream_t s) {
   // prompts does not pass): sequences with one query token go to the decode kernel, which reads their
   // K/V once for all heads of a group instead of walking them in 64-row tiles with one row in use.
   // 3 chunks of 512 tokens and 45 decode tokens over 192 thousand keys, 32/8 heads, D 128: 197 us with
-  // all of them as tiles, 147 us with the decode kernel in front of this one, 135 us behind it.
-  const int skip_single = p->total_q > 0 && p->q_start != p->k_start && p->causal && p->fine_block == 0 &&
-                          p->row_mode == BSA_ROWS_BY_POSITION && (p->d == 64 || p->d == 128) && p->batch <= 65535;
+  // all of them as tiles, 147 us with the decode kernel in front of this one, 130 us behind it.
+  // How many there are stands on the device only, and where there are none the launch costs 0.6 to 1 us
+  // for nothing.  So not where as many queries as keys say whole prompts, nor below four sequences, where
+  // it is a tenth of a small call (a chunk of 64: 8.5 -> 9.3 us) and one to three tokens fit beside the
+  // tiles (chunk of 512 + 1 token: 29.8 us either way; + 3 tokens: 32.6 as tiles, 29.8 with the launch).
+  const int skip_single = p->total_q > 0 && p->q_start != p->k_start && p->total_q != p->sk && p->batch >= 4 &&
+                          p->batch <= 65535 && p->causal && p->fine_block == 0 &&
+                          p->row_mode == BSA_ROWS_BY_POSITION && (p->d == 64 || p->d == 128);
   const int rc = launch_fwd_for(p, zero_pads, skip_single, s);
   return rc || !skip_single ? rc : decode_packed_rows(p, s);
 }

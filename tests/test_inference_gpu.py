@@ -586,3 +586,44 @@ def test_pad_rows_of_empty_sequences_and_of_unaligned_outputs(Hq, Hkv, D, extra)
     pad = torch.arange(S, device="cuda")[None] < left[:, None]
     assert (o[pad] == 0).all() and torch.isneginf(lse.transpose(1, 2)[pad]).all()
     assert (buf[..., D:] == 7.0).all()
+
+
+def _launches(fn):
+    """Number of nodes of the graph that a call of fn is captured into."""
+    import ctypes
+    fn()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    n = ctypes.c_size_t(0)
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(g.raw_cuda_graph()), None, ctypes.byref(n)) == 0
+    return n.value
+
+
+@pytest.mark.parametrize("q_lens,k_lens,second", [
+    ([64], [192], False),                                  # one chunk
+    ([65, 1, 1], [193, 700, 33], False),                   # too few sequences
+    ([1, 64, 130, 1], [1, 64, 130, 1], False),             # whole prompts (as many queries as keys)
+    ([65, 1, 0, 1], [193, 700, 0, 33], True),
+    ([64, 64, 64, 64, 64], [64, 128, 192, 256, 320], True),   # chunks only: the launch finds nothing to do
+    ([1, 1, 1, 1, 1], [1, 64, 65, 128, 511], True),           # no tile at all
+])
+def test_packed_call_launches_the_single_token_kernel_where_it_pays(q_lens, k_lens, second):
+    """A packed batch whose query ranges cannot hold single decode tokens, or few of them, is one launch; both routes
+    give the oracle's rows, and what follows in the stream sees them."""
+    Hq, Hkv, D, bs, S = 8, 2, 64, 64, 1024
+    pk = dict(block_size=bs, local_blocks=3, vert_stride=4, num_kv_heads=Hkv)
+    mod = _module(Hq, S, pk, impl="sm100")
+    cu_q = torch.tensor(np.cumsum([0] + q_lens), dtype=torch.int32)
+    cu_k = torch.tensor(np.cumsum([0] + k_lens), dtype=torch.int32)
+    q, k, v = seeded_qkv(99, (sum(q_lens), Hq, D), (sum(k_lens), Hkv, D), torch.bfloat16)
+    ref, ref_lse = O.varlen_attention(q.float(), k.float(), v.float(), cu_k, O.block_mask(Hq, S, **pk), bs, cu_seqlens_q=cu_q)
+    q, k, v, cu_q, cu_k = (t.cuda() for t in (q, k, v, cu_q, cu_k))
+
+    def call(return_lse=False):
+        with torch.no_grad():
+            return mod(q, k, v, cu_seqlen_k=cu_k, cu_seqlen_q=cu_q, return_lse=return_lse)
+    out, lse = call(True)
+    assert_out_close(out.clone(), ref)
+    assert_lse_close(lse, ref_lse)
+    assert _launches(call) == (2 if second else 1)
