@@ -76,6 +76,11 @@ template <> struct MmaType<__half> {
     __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
   }
+  // what the packed pair leaves of its two sources
+  static __device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t packed) {
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&packed));
+    return pack(lo - h.x, hi - h.y);
+  }
 };
 template <> struct MmaType<__nv_bfloat16> {
   static __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
@@ -89,6 +94,9 @@ template <> struct MmaType<__nv_bfloat16> {
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
+  }
+  static __device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t packed) {
+    return pack(lo - __uint_as_float(packed << 16), hi - __uint_as_float(packed & 0xffff0000u));
   }
 };
 
@@ -176,18 +184,27 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
 
 // NT: 8-column tiles of q heads (heads_per_cta <= 8 NT).
 //
+// P enters V^T P^T as two 16-bit terms, P = hi + lo, which keeps its fp32 value to 2^-16 (bf16) or better.
+// One term rounds every weight at 2^-9 (bf16) or 2^-12 (f16), and a reference maximum that is raised lazily
+// leaves not even a row's largest weights exact: error against 64 bits, apart from the rounding of the output,
+// 1.53e-3 of the output with bf16 and 1.8e-4 with e4m3 K/V, now 2.4e-6 and 2.5e-7.  FOLD: where the last
+// tile holds up to four heads, their lo terms take its columns 4..7 (its q rows 4..7 repeat rows 0..3, so that
+// the logits are there already) and cost no product of their own (the e4m3 step below 53.0 instead of 55.7 us);
+// those of a fuller tile are a second product on the same V fragments.
+//
 // Bound by HBM with a 16-bit cache; with an 8-bit cache by the fixed cost of a CTA (row lookup, first
 // tiles, merge of the warps: 7 us) and the latency of a unit.  64 sequences of 1024..8192 tokens, 32/8
-// heads, D 128, local 16 + stride 8, with the merge kernel: 69 us for the 401 MB of a bf16 cache, 54 us for
-// the 203 MB of an e4m3 cache.  (78 and 79 us when all four warps shared a unit, 16 tokens each, with the
+// heads, D 128, local 16 + stride 8, with the merge kernel: 68 us for the 401 MB of a bf16 cache, 53 us for
+// the 203 MB of an e4m3 cache (67.5 and 52.4 with P in one term).  (78 and 79 us when all four warps shared a unit, 16 tokens each, with the
 // heads on the rows; 71 and 56 us when a producer warp refilled K and V together after both were read.)
-template <typename T, int D, bool FP8, int NT>
+template <typename T, int D, bool FP8, int NT, bool FOLD>
 __global__ void __launch_bounds__(kDecThreads, FP8 && D == 128 && NT == 2 ? 2 : kMinCtas)   // 2: spills otherwise
 decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 tmV,
               bsa_decode_params p, int nsplit, int cl, int max_units, const int32_t* __restrict__ row_start,
               const int32_t* __restrict__ row_end, int* wait_status) {
   using Geo = DecGeo<D, FP8>;
   constexpr int kStages = Geo::kStages, kTok = Geo::kTok;
+  constexpr int kLoTiles = FOLD ? NT - 1 : NT;   // column tiles whose lo terms are a product of their own
   constexpr int kTileBytes = Geo::kTileBytes;
   constexpr int kStageBytes = Geo::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
@@ -311,11 +328,12 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       for (int u = 0; u < nu && u < kStages; ++u) load_tile(u, true);
     }
   } else {
-    // q heads of the group -> rows of the q tile (rows >= GH are zero), 16 bytes a thread.  The maximum is
+    // q heads of the group -> rows of the q tile (rows of no head are zero), 16 bytes a thread.  The maximum is
     // taken and the end of the sequence masked before the logits are scaled, which asks for a positive
     // scale: a negative one hands its sign to q here, and scale 0 makes the products themselves zero.
     for (int i = tid; i < NT * 8 * D / 8; i += kConsumers * 32) {
-      const int r = i / (D / 8), c = i % (D / 8);
+      const int row = i / (D / 8), c = i % (D / 8);
+      const int r = FOLD && row >= NT * 8 - 4 ? row - 4 : row;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (r < GH) {
         const T* src = reinterpret_cast<const T*>(p.q) + (int64_t)qb * p.q_sb + (int64_t)(h0 + r) * p.q_sh + c * 8;
@@ -488,8 +506,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
           }
         }
       }
-      // P^T as the B operand: the 8x8 tiles of S^T's accumulator layout, transposed
-      uint32_t pb[kTok / 16][NT][2];
+      // P^T as the B operand: the 8x8 tiles of S^T's accumulator layout, transposed; FOLD: lo in columns 4..7 of the last tile
+      uint32_t pb[kTok / 16][NT][2], pl[kTok / 16][NT][2];
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
         const float n0 = m[nt][0] == -INFINITY ? 0.f : -m[nt][0], n1 = m[nt][1] == -INFINITY ? 0.f : -m[nt][1];
@@ -499,8 +517,14 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
           const float p2 = dec_ex2(fmaf(sacc[mt][nt][2], mul, n0)), p3 = dec_ex2(fmaf(sacc[mt][nt][3], mul, n1));
           l[nt][0] += p0 + p2;
           l[nt][1] += p1 + p3;
-          pb[mt][nt][0] = transpose8x8(MmaType<MT>::pack(p0, p1));
-          pb[mt][nt][1] = transpose8x8(MmaType<MT>::pack(p2, p3));
+          const uint32_t hi0 = MmaType<MT>::pack(p0, p1), hi1 = MmaType<MT>::pack(p2, p3);
+          const uint32_t lo0 = MmaType<MT>::pack_rest(p0, p1, hi0), lo1 = MmaType<MT>::pack_rest(p2, p3, hi1);
+          pb[mt][nt][0] = transpose8x8(FOLD && nt == NT - 1 && tq >= 2 ? lo0 : hi0);
+          pb[mt][nt][1] = transpose8x8(FOLD && nt == NT - 1 && tq >= 2 ? lo1 : hi1);
+          if (nt < kLoTiles) {
+            pl[mt][nt][0] = transpose8x8(lo0);
+            pl[mt][nt][1] = transpose8x8(lo1);
+          }
         }
       }
       if (!mbar_wait(&sm->v_full[s], ph, wait_status, 101)) break;
@@ -545,6 +569,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
             cvt_e4m3x4(byte_perm(rows[2][wi], rows[3][wi], sel), a[2], a[3]);   // tokens 8+2tq, 9+2tq
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) MmaType<MT>::mma(oacc[md][nt], a, pb[mt][nt][0], pb[mt][nt][1]);
+#pragma unroll
+            for (int nt = 0; nt < kLoTiles; ++nt) MmaType<MT>::mma(oacc[md][nt], a, pl[mt][nt][0], pl[mt][nt][1]);
           }
         } else {
 #pragma unroll
@@ -554,6 +580,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
             ldsm_x4_t(vbase + Geo::off(mt * 16 + (j >> 1) * 8 + (lane & 7), md * 2 + (j & 1)), a[0], a[1], a[2], a[3]);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) MmaType<MT>::mma(oacc[md][nt], a, pb[mt][nt][0], pb[mt][nt][1]);
+#pragma unroll
+            for (int nt = 0; nt < kLoTiles; ++nt) MmaType<MT>::mma(oacc[md][nt], a, pl[mt][nt][0], pl[mt][nt][1]);
           }
         }
       }
@@ -636,7 +664,11 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
 #pragma unroll
     for (int w = 0; w < kConsumers; ++w) {
       const float sc = exp2f(sm->wm[w][r] - msafe);
-      const float4 v = *reinterpret_cast<const float4*>(Om + (w * NT * 8 + r) * kRow + d);
+      float4 v = *reinterpret_cast<const float4*>(Om + (w * NT * 8 + r) * kRow + d);
+      if (FOLD && (NT == 1 || r >= 8)) {   // the lo terms' part
+        const float4 lo = *reinterpret_cast<const float4*>(Om + (w * NT * 8 + r + 4) * kRow + d);
+        v.x += lo.x; v.y += lo.y; v.z += lo.z; v.w += lo.w;
+      }
       acc.x += v.x * sc; acc.y += v.y * sc; acc.z += v.z * sc; acc.w += v.w * sc;
       l += sm->wl[w][r] * sc;
     }
@@ -769,7 +801,7 @@ int decode_nsplit(const bsa_decode_params* p) {
   return n < 1 ? 1 : n;
 }
 
-template <typename T, int D, bool FP8, int NT>
+template <typename T, int D, bool FP8, int NT, bool FOLD>
 int launch_decode(const bsa_decode_params* p, int nsplit, int cl, const int32_t* row_start, const int32_t* row_end,
                   cudaStream_t s) {
   Tmap4 tmK, tmV;
@@ -787,7 +819,7 @@ int launch_decode(const bsa_decode_params* p, int nsplit, int cl, const int32_t*
   q.blocks_per_split = decode_blocks_per_split(p);
   const int max_units = q.blocks_per_split * (p->block_size / Geo::kTok);
   const size_t smem = dec_smem<D, FP8, NT>(max_units);
-  auto kern = decode_kernel<T, D, FP8, NT>;
+  auto kern = decode_kernel<T, D, FP8, NT, FOLD>;
   // one value for every call: host threads may launch this kernel with different sizes at the same time
   BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)dec_smem<D, FP8, NT>(kMaxRowBlocks * 64 / Geo::kTok)));
@@ -834,12 +866,18 @@ template <typename T>
 int launch_decode_t(const bsa_decode_params* p, bool fp8, int nsplit, int cl, const int32_t* row_start,
                     const int32_t* row_end, cudaStream_t s) {
   auto go = [&](auto kernel) { return kernel(p, nsplit, cl, row_start, row_end, s); };
-  if (p->heads_per_cta > 8) {
-    if (fp8) return p->d == 128 ? go(launch_decode<T, 128, true, 2>) : go(launch_decode<T, 64, true, 2>);
-    return p->d == 128 ? go(launch_decode<T, 128, false, 2>) : go(launch_decode<T, 64, false, 2>);
-  }
-  if (fp8) return p->d == 128 ? go(launch_decode<T, 128, true, 1>) : go(launch_decode<T, 64, true, 1>);
-  return p->d == 128 ? go(launch_decode<T, 128, false, 1>) : go(launch_decode<T, 64, false, 1>);
+  auto go_heads = [&](auto d, auto kv8) {
+    constexpr int D = decltype(d)::value;
+    constexpr bool FP8 = decltype(kv8)::value;
+    if (p->heads_per_cta > 12) return go(launch_decode<T, D, FP8, 2, false>);
+    if (p->heads_per_cta > 8) return go(launch_decode<T, D, FP8, 2, true>);
+    if (p->heads_per_cta > 4) return go(launch_decode<T, D, FP8, 1, false>);
+    return go(launch_decode<T, D, FP8, 1, true>);
+  };
+  using D64 = std::integral_constant<int, 64>;
+  using D128 = std::integral_constant<int, 128>;
+  if (fp8) return p->d == 128 ? go_heads(D128(), std::true_type()) : go_heads(D64(), std::true_type());
+  return p->d == 128 ? go_heads(D128(), std::false_type()) : go_heads(D64(), std::false_type());
 }
 
 }  // namespace

@@ -627,3 +627,34 @@ def test_packed_call_launches_the_single_token_kernel_where_it_pays(q_lens, k_le
     assert_out_close(out.clone(), ref)
     assert_lse_close(lse, ref_lse)
     assert _launches(call) == (2 if second else 1)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,D,dtype", [
+    (3, 1, 128, torch.bfloat16), (8, 2, 64, torch.bfloat16), (4, 4, 128, torch.float16),      # lo terms in idle columns
+    (6, 1, 64, torch.float16), (8, 1, 128, torch.bfloat16),                                    # ... as a second product
+    (12, 1, 128, torch.bfloat16), (9, 1, 64, torch.float16), (16, 1, 64, torch.float16),        # two column tiles
+])
+def test_decode_weights_keep_their_fp32_value(fp8, Hq, Hkv, D, dtype):
+    """fp32 partials (no rounding of the output) against 64 bits.  Two 16-bit terms leave 2^-18 of a weight, the
+    fp32 logits (up to 2^4) and exponentials a few 2^-20; one term alone would show 2^-9 / sqrt(3) = 1.1e-3 (bf16)
+    or 1.4e-4 (f16)."""
+    from dkernel_b200.ops import decode
+    bs, lens = 64, [1, 63, 64, 200, 777, 1024]
+    B, S = len(lens), 1024
+    pk = dict(block_size=bs, local_blocks=16, vert_stride=4, num_kv_heads=Hkv)      # dense rows of 16 blocks
+    q, k, v = (t.cuda() for t in seeded_qkv(101, (B, 1, Hq, D), (B, S, Hkv, D), dtype))
+    scales, kw = (1.0, 1.0), {}
+    if fp8:
+        scales = (0.02, 0.015)
+        k, v, kw = (k.float() / scales[0]).to(torch.float8_e4m3fn), (v.float() / scales[1]).to(torch.float8_e4m3fn), dict(kv_scales=scales)
+    left = torch.tensor([S - n for n in lens], dtype=torch.int32, device="cuda")
+    o, _ = decode(q, k, v, _module(Hq, S, pk, seq_dim=1)._plan(), 1.0 / math.sqrt(D), seq_dim=1, k_start=left,
+                  blocks_per_split=16, partials_only=True, **kw)
+    k, v = (t.double().repeat_interleave(Hq // Hkv, 2) * s for t, s in zip((k, v), scales))
+    ref = torch.empty(B, Hq, D, dtype=torch.float64, device="cuda")
+    for i, n in enumerate(lens):
+        p = torch.softmax(torch.einsum("hd,nhd->hn", q[i, 0].double(), k[i, S - n:]) / math.sqrt(D), -1)
+        ref[i] = torch.einsum("hn,nhd->hd", p, v[i, S - n:])
+    err = (o.view(B, Hq, D).double() - ref).norm() / ref.norm()
+    assert err <= 2e-5, float(err)
