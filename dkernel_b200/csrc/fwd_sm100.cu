@@ -27,6 +27,7 @@ constexpr int kBS = 64;
 constexpr int kThreadsP = 224;
 constexpr int kWarpProd = 4, kWarpIssue = 5, kWarpPlan = 6;
 constexpr int kMaxList = 1024;           // kv blocks per sequence (64K tokens)
+constexpr uint32_t kBlkMask = kMaxList - 1;   // the block of a list entry
 // Shared-memory tiles are stored as D/64 sub-tiles of [rows][128 bytes] (one TMA box each,
 // 128-byte swizzled): Q 128 rows (16 KB per sub-tile), K and V 64 rows (8 KB per sub-tile).
 template <int D> struct Geo {
@@ -43,9 +44,12 @@ struct Plan {
   int n;                     // number of kv blocks in list
   int b, kvh;
   int head[2], qblk[2], hvalid[2];
-  int cbeg[2];               // first CSR entry of each half's pattern row (fine-block patterns)
+  // fine-block patterns: the sub-row of its pattern row that each half starts at, the first CSR entry of that row
+  // and, where the half reaches into it, of the next
+  int sub0[2], cbeg[2], cnext[2];
   int q_start, q_len, k_start, k_len, past;
-  uint16_t list[kMaxList];   // block | attended-by-half-0 << 14 | attended-by-half-1 << 15
+  uint16_t list[kMaxList];   // block | attended-by-half-0 << 14 | attended-by-half-1 << 15; fine-block patterns:
+                             // block | attended by half t's first (second) pattern row << 10 (12) + t
 };
 
 struct TailP {
@@ -57,7 +61,7 @@ struct TailP {
   uint64_t qk_done[2], p_full[2], pv_done[2];
   uint64_t o_free;           // the epilogue has read O
   uint32_t tmem_base;
-  uint32_t bits[2][kMaxList / 32];
+  uint32_t bits[4][kMaxList / 32];   // by half; 2, 3: second pattern rows
   Plan plan[2];
   // epilogue: 32 rows x 64 bytes per softmax warp, so that a store instruction covers whole
   // 64-byte row pieces of eight rows instead of 16 bytes of thirty-two rows
@@ -89,6 +93,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 
 // item -> plan (executed by the whole planner warp)
 // Returns false when no sequence has this tile, nor any tile of a later item.
+template <int FB>
 __device__ __forceinline__ bool build_plan(const bsa_fwd_params& p, int mode, int item, int tiles_x,
                                            int head_items, bool skip_single, Plan* pl, uint32_t (*bits)[kMaxList / 32],
                                            int lane, int* wait_status) {
@@ -152,35 +157,42 @@ __device__ __forceinline__ bool build_plan(const bsa_fwd_params& p, int mode, in
     hvalid[1] = valid && qblk[1] * kBS < q_len;
   }
   const int nkb = min((k_len + kBS - 1) / kBS, kMaxList);
-  bits[0][lane] = 0u;
-  bits[1][lane] = 0u;
-  int cbeg[2] = {0, 0};
+#pragma unroll
+  for (int i = 0; i < (FB ? 4 : 2); ++i) bits[i][lane] = 0u;
+  int sub0[2] = {0, 0}, cbeg[2][2] = {};
   __syncwarp();
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
     if (!hvalid[t]) continue;
     const int q_first = qblk[t] * kBS;
-    const int row = (p.row_mode == BSA_ROWS_BY_POSITION ? past + q_first : q_first) / kBS;
-    if (row >= p.n_rows) continue;
+    const int pos = p.row_mode == BSA_ROWS_BY_POSITION ? past + q_first : q_first;
+    const int q_pos_last = past + min(q_first + kBS, q_len) - 1;
     const int hp = pattern_head(head[t], p.h_pat, p.hq, p.hkv);
     const int32_t* cr = p.crow + (int64_t)hp * p.crow_sh;
     const int32_t* cols = p.col + (int64_t)hp * p.col_sh;
-    const int c_beg = __ldg(cr + row), c_end = __ldg(cr + row + 1);
-    cbeg[t] = c_beg;
-    // a CSR row is a range of its head's column array
-    if (!BSA_IN_BOUNDS(c_beg >= 0 && c_beg <= c_end && (p.col_sh == 0 || c_end <= p.col_sh), wait_status, 801))
-      continue;
-    const int q_pos_last = past + min(q_first + kBS, q_len) - 1;
-    for (int i = c_beg + lane; i < c_end; i += 32) {
-      const int blk = __ldg(cols + i);
-      if (blk >= 0 && blk < nkb && !(p.causal && blk * kBS > q_pos_last))
-        atomicOr(&bits[t][blk >> 5], 1u << (blk & 31));
+    // Positions need not start on a 64-token boundary (a decode token never has to): the half's sub-blocks then
+    // begin inside one row of the coarsened pattern and go on in the next.
+    if (FB) sub0[t] = (pos % kBS) / (FB ? FB : 1);
+#pragma unroll
+    for (int x = 0; x < (FB ? 2 : 1); ++x) {
+      const int row = pos / kBS + x;
+      if (row >= p.n_rows || (x && min(q_len - q_first, kBS) <= kBS - sub0[t] * FB)) break;
+      const int c_beg = __ldg(cr + row), c_end = __ldg(cr + row + 1);
+      cbeg[t][x] = c_beg;
+      // a CSR row is a range of its head's column array
+      if (!BSA_IN_BOUNDS(c_beg >= 0 && c_beg <= c_end && (p.col_sh == 0 || c_end <= p.col_sh), wait_status, 801))
+        continue;
+      for (int i = c_beg + lane; i < c_end; i += 32) {
+        const int blk = __ldg(cols + i);
+        if (blk >= 0 && blk < nkb && !(p.causal && blk * kBS > q_pos_last))
+          atomicOr(&bits[t + 2 * x][blk >> 5], 1u << (blk & 31));
+      }
     }
   }
   __syncwarp();
   // bitmaps -> ordered list: scan the word counts, then every lane owns one bit of a word
   const uint32_t u0 = bits[0][lane], u1 = bits[1][lane];
-  const uint32_t u = u0 | u1;
+  const uint32_t u = u0 | u1 | (FB ? bits[FB ? 2 : 0][lane] | bits[FB ? 3 : 0][lane] : 0u);
   const int cnt = __popc(u);
   int incl = cnt;
 #pragma unroll
@@ -194,12 +206,19 @@ __device__ __forceinline__ bool build_plan(const bsa_fwd_params& p, int mode, in
     const int w = __ffs(nonzero) - 1;
     nonzero &= nonzero - 1;
     const uint32_t uw = __shfl_sync(0xffffffffu, u, w);
-    const uint32_t u0w = __shfl_sync(0xffffffffu, u0, w);
-    const uint32_t u1w = __shfl_sync(0xffffffffu, u1, w);
     const int bw = __shfl_sync(0xffffffffu, base, w);
+    uint32_t flags;
+    if (FB) {
+      flags = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) flags |= ((bits[FB ? i : 0][w] >> lane) & 1u) << (10 + i);
+    } else {
+      const uint32_t u0w = __shfl_sync(0xffffffffu, u0, w);
+      const uint32_t u1w = __shfl_sync(0xffffffffu, u1, w);
+      flags = (((u0w >> lane) & 1u) << 14) | (((u1w >> lane) & 1u) << 15);
+    }
     if (((uw >> lane) & 1u) && BSA_IN_BOUNDS(bw + __popc(uw & ((1u << lane) - 1u)) < kMaxList, wait_status, 802))
-      pl->list[bw + __popc(uw & ((1u << lane) - 1u))] =
-          (uint16_t)((w * 32 + lane) | (((u0w >> lane) & 1u) << 14) | (((u1w >> lane) & 1u) << 15));
+      pl->list[bw + __popc(uw & ((1u << lane) - 1u))] = (uint16_t)((w * 32 + lane) | flags);
   }
   const int n = __shfl_sync(0xffffffffu, incl, 31);
   if (lane == 0) {
@@ -210,7 +229,10 @@ __device__ __forceinline__ bool build_plan(const bsa_fwd_params& p, int mode, in
     pl->head[0] = head[0]; pl->head[1] = head[1];
     pl->qblk[0] = qblk[0]; pl->qblk[1] = qblk[1];
     pl->hvalid[0] = hvalid[0]; pl->hvalid[1] = hvalid[1];
-    pl->cbeg[0] = cbeg[0]; pl->cbeg[1] = cbeg[1];
+    if (FB) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) { pl->sub0[t] = sub0[t]; pl->cbeg[t] = cbeg[t][0]; pl->cnext[t] = cbeg[t][1]; }
+    }
     pl->q_start = q_start; pl->q_len = q_len; pl->k_start = k_start; pl->k_len = k_len;
     pl->past = past;
   }
@@ -318,7 +340,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
       const int pb = k & 1;
       if (!mbar_wait(&tl->plan_free[pb], ((k >> 1) & 1) ^ 1, wait_status, 401)) break;
       if (item >= n_items || item < 0 ||
-          !build_plan(p, mode, item, tiles_x, head_items, skip_single, &tl->plan[pb], tl->bits, lane, wait_status)) {
+          !build_plan<FB>(p, mode, item, tiles_x, head_items, skip_single, &tl->plan[pb], tl->bits, lane, wait_status)) {
         if (lane == 0) {
           tl->plan[pb].valid = -1;
           tl->plan[pb].n = 0;
@@ -374,7 +396,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
           auto load_k = [&](int j) -> bool {
             const uint32_t gk = g + (uint32_t)j;
             const int s = gk & 1;
-            const int tok = pl->k_start + (int)(pl->list[j] & 0x3fffu) * kBS;
+            const int tok = pl->k_start + (int)(pl->list[j] & kBlkMask) * kBS;
             uint8_t* kdst = sRing + s * 2 * kTile;
             // a listed block starts inside the stored keys of its kv head (its tail may be past them)
             (void)BSA_IN_BOUNDS(tok >= 0 && tok < p.sk && pl->kvh >= 0 && pl->kvh < p.hkv, wait_status, 804);
@@ -390,7 +412,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
             if (j + 1 < n && !load_k(j + 1)) { ok = false; break; }
             const uint32_t gv = g + (uint32_t)j;
             const int s = gv & 1;
-            const int tok = pl->k_start + (int)(pl->list[j] & 0x3fffu) * kBS;
+            const int tok = pl->k_start + (int)(pl->list[j] & kBlkMask) * kBS;
             if (!mbar_wait(&tl->pv_done[s], ((gv >> 1) & 1) ^ 1, wait_status, 405)) { ok = false; break; }
             mbar_expect_tx(&tl->v_full[s], kTile);
 #pragma unroll
@@ -515,24 +537,29 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
         continue;
       }
       float m_used = -INFINITY, l = 0.f;
-      // fine-block patterns: this half's entries of the tile are a prefix of its CSR row, in order
+      // fine-block patterns: the entries that this thread's row attends are a prefix of a CSR row, in order
       constexpr int kF = FB ? kBS / FB : 1;                  // sub-blocks per side
       constexpr uint32_t kFull = (1u << kF) - 1u;
       const int32_t* fbits = nullptr;
+      int sub = 0, flag = 14 + t;                            // sub-row of the pattern row; its bit in a list entry
       if (FB) {
         const int hp = pattern_head(head, p.h_pat, p.hq, p.hkv);
-        fbits = p.col_bits + (int64_t)hp * p.col_bits_sh + pl->cbeg[t];
+        sub = pl->sub0[t] + rr / (FB ? FB : 1);
+        const bool next = sub >= kF;
+        if (next) sub -= kF;
+        flag = (next ? 12 : 10) + t;
+        fbits = p.col_bits + (int64_t)hp * p.col_bits_sh + (next ? pl->cnext[t] : pl->cbeg[t]);
       }
       for (int j = 0; j < n; ++j, ++g) {
         const int s = g & 1;
         // everything that only depends on the block list is done before the barrier probe
         const uint32_t ent = pl->list[j];
-        const int kbase = (int)(ent & 0x3fffu) * kBS;
-        const bool att = ((ent >> (14 + t)) & 1u) != 0 && hvalid;
+        const int kbase = (int)(ent & kBlkMask) * kBS;
+        const bool att = ((ent >> flag) & 1u) != 0 && hvalid;
         int lim = k_len - kbase;
         if (p.causal) lim = min(lim, qpos - kbase + 1);
         uint32_t cm = kFull;     // which sub-columns this row attends inside the block
-        if (FB && att) cm = ((uint32_t)__ldg(fbits++) >> ((rr / (FB ? FB : 1)) * kF)) & kFull;
+        if (FB && att) cm = ((uint32_t)__ldg(fbits++) >> (sub * kF)) & kFull;
         // the entries of this half that the tile walks are a prefix of its CSR row
         if (FB && att)
           (void)BSA_IN_BOUNDS(p.col_bits_sh == 0 || fbits - p.col_bits - (int64_t)pattern_head(head, p.h_pat, p.hq, p.hkv) *

@@ -658,3 +658,26 @@ def test_decode_weights_keep_their_fp32_value(fp8, Hq, Hkv, D, dtype):
         ref[i] = torch.einsum("hn,nhd->hd", p, v[i, S - n:])
     err = (o.view(B, Hq, D).double() - ref).norm() / ref.norm()
     assert err <= 2e-5, float(err)
+
+
+@pytest.mark.parametrize("many_keys", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,D,bs,dtype", [(4, 2, 64, 32, torch.bfloat16), (3, 3, 128, 16, torch.float16),
+                                               (2, 2, 64, 16, torch.bfloat16), (4, 1, 128, 32, torch.float16)])
+def test_packed_fine_blocks_from_any_position(Hq, Hkv, D, bs, dtype, many_keys):
+    """Decode tokens and chunks of 16- and 32-token patterns that do not start on a 64-token boundary: a tile's
+    sub-blocks then lie in two rows of the coarsened pattern, the last of them behind its end."""
+    S = 5120
+    pk = dict(block_size=bs, local_blocks=2, vert_stride=3, num_kv_heads=Hkv)
+    starts = [0, bs, 64 - bs, 64, 3 * bs, 64 + bs, 5 * bs, 7 * bs] + [4096 + bs] * (16 if many_keys else 0)
+    q_lens = [1, 64, 130, 1, 63, 1, bs, 200] + [1] * (16 if many_keys else 0)
+    k_lens = [a + n for a, n in zip(starts, q_lens)]
+    q_lens, k_lens = q_lens + [1, 1, 64], k_lens + [48, 333, S]
+    assert (sum(k_lens) > 65536) == many_keys
+    cu_q, cu_k = (torch.tensor(np.cumsum([0] + n), dtype=torch.int32) for n in (q_lens, k_lens))
+    q, k, v = seeded_qkv(107, (sum(q_lens), Hq, D), (sum(k_lens), Hkv, D), dtype)
+    ref, ref_lse = O.varlen_attention(q.float(), k.float(), v.float(), cu_k, O.block_mask(Hq, S, **pk), bs, cu_seqlens_q=cu_q)
+    mod = _module(Hq, S, pk, impl="sm100")
+    with torch.no_grad():
+        out, lse = mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda(), return_lse=True)
+    assert_out_close(out, ref)
+    assert_lse_close(lse, ref_lse)
