@@ -91,6 +91,21 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
+// what the 16-bit pair `hi` leaves of lo, hi's sources: the second term of P = P_hi + P_lo
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2_rest(float p0, float p1, uint32_t hi) {
+  float h0, h1;
+  if (BF16) {
+    h0 = __uint_as_float(hi << 16);
+    h1 = __uint_as_float(hi & 0xffff0000u);
+  } else {
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    h0 = h.x;
+    h1 = h.y;
+  }
+  return pack2<BF16>(p0 - h0, p1 - h1);
+}
+
 // item -> plan (executed by the whole planner warp)
 // Returns false when no sequence has this tile, nor any tile of a later item.
 template <int FB>
@@ -267,7 +282,11 @@ __device__ __forceinline__ void store_pad_rows(const bsa_fwd_params& p, int head
 // FB: 0, or the pattern's own block size (16 or 32) when it is finer than the 64-token tiles: the
 // CSR then describes the pattern coarsened to 64 x 64 blocks and col_bits holds, per CSR entry,
 // one bit per (sub-row, sub-column) pair of the block (bit a * (64/FB) + b).
-template <bool BF16, int D, int FB>
+// SPLIT: P = hi + lo, two 16-bit terms side by side in S's columns and 128 instead of 64 "tokens" for
+// P V, the second half on the same V rows.  Error against 64 bits apart from the rounding of the output,
+// chunks beside decode tokens, bf16: 1.6e-3 of the output with one term, 4e-6 with two (fp32 arithmetic on
+// the CUDA cores: 7e-7); the call as a whole 130 -> 145 us (12.6 ms there).
+template <bool BF16, int D, int FB, bool SPLIT>
 __global__ void __launch_bounds__(kThreadsP, D <= 128 ? 2 : 1)
 fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tmap4 tmK,
                    const __grid_constant__ Tmap4 tmV, bsa_fwd_params p, int mode, int n_items,
@@ -478,8 +497,8 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
           const uint32_t acc0 = j ? 1u : 0u;
           if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              tc_mma_ts(tO, tS[s] + kk * 8, dv0 + (uint64_t)((kk * 2048) >> 4), idesc_pv, kk ? 1u : acc0);
+            for (int kk = 0; kk < (SPLIT ? 8 : 4); ++kk)   // 4..7: the low parts of P
+              tc_mma_ts(tO, tS[s] + kk * 8, dv0 + (uint64_t)(((kk & 3) * 2048) >> 4), idesc_pv, kk ? 1u : acc0);
             tc_commit(&tl->pv_done[s]);
           }
           __syncwarp();
@@ -640,7 +659,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
         uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
         for (int hlf = 0; hlf < 2; ++hlf) {
-          uint32_t pk[16];
+          uint32_t pk[16], pl[SPLIT ? 16 : 1];
           if (live && (FB != 32 || ((cm >> hlf) & 1u))) {
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
@@ -649,12 +668,16 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
               const float p0 = ex2(x0), p1 = ex2(x1);
               sum2[c & 1] = add_f32x2(sum2[c & 1], f32x2(p0, p1));
               pk[c] = pack2<BF16>(p0, p1);
+              if (SPLIT) pl[SPLIT ? c : 0] = pack2_rest<BF16>(p0, p1, pk[c]);
             }
           } else {
 #pragma unroll
             for (int c = 0; c < 16; ++c) pk[c] = 0u;
+#pragma unroll
+            for (int c = 0; c < (SPLIT ? 16 : 1); ++c) pl[c] = 0u;
           }
           tmem_st16(tS[s] + lane_off + hlf * 16, pk);
+          if constexpr (SPLIT) tmem_st16(tS[s] + lane_off + 32 + hlf * 16, pl);
         }
         float sum[4];
         f32x2_split(sum2[0], sum[0], sum[1]);
@@ -784,7 +807,11 @@ bool sm100_fwd_supported(const bsa_fwd_params* p, const char** why) {
 }
 
 namespace {
-template <bool BF16, int D, int FB>
+// More than 65536 keys, which only a packed batch has here: such calls ran on the CUDA-core kernel, whose
+// weights are fp32 throughout, before this kernel took them; with P in two terms it is no less precise.
+bool split_p(const bsa_fwd_params* p) { return p->sk > kMaxList * kBS; }
+
+template <bool BF16, int D, int FB, bool SPLIT>
 int launch_fwd(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStream_t s) {
   Tmap4 tmQ, tmK, tmV;
   const uint64_t nb = p->total_q > 0 ? 1 : p->batch;
@@ -820,25 +847,27 @@ int launch_fwd(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStre
   int* status = wait_status_ptr();
   if (!status) return BSA_E_CUDA;
   constexpr size_t smem = Geo<D>::kSmem + sizeof(TailP);
-  auto kern = fwd_persist_kernel<BF16, D, FB>;
+  auto kern = fwd_persist_kernel<BF16, D, FB, SPLIT>;
   BSA_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<grid, kThreadsP, smem, s>>>(tmQ, tmK, tmV, *p, mode, n_items, tiles_x, head_items, zero_pads, skip_single,
                                      status);
   return check_launch("fwd_persist_kernel");
 }
-int launch_fwd_for(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStream_t s) {
-  const bool bf16 = p->dtype == BSA_BF16;
-  if (p->fine_block == 16) {
-    if (p->d <= 64) return bf16 ? launch_fwd<true, 64, 16>(p, zero_pads, skip_single, s) : launch_fwd<false, 64, 16>(p, zero_pads, skip_single, s);
-    return bf16 ? launch_fwd<true, 128, 16>(p, zero_pads, skip_single, s) : launch_fwd<false, 128, 16>(p, zero_pads, skip_single, s);
+template <bool BF16, int FB>
+int launch_fwd_d(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStream_t s) {
+  const bool split = split_p(p);
+  auto go = [&](auto one, auto two) { return (split ? two : one)(p, zero_pads, skip_single, s); };
+  if (p->d <= 64) return go(launch_fwd<BF16, 64, FB, false>, launch_fwd<BF16, 64, FB, true>);
+  if constexpr (FB == 0) {
+    if (p->d > 128) return go(launch_fwd<BF16, 256, 0, false>, launch_fwd<BF16, 256, 0, true>);
   }
-  if (p->fine_block == 32) {
-    if (p->d <= 64) return bf16 ? launch_fwd<true, 64, 32>(p, zero_pads, skip_single, s) : launch_fwd<false, 64, 32>(p, zero_pads, skip_single, s);
-    return bf16 ? launch_fwd<true, 128, 32>(p, zero_pads, skip_single, s) : launch_fwd<false, 128, 32>(p, zero_pads, skip_single, s);
-  }
-  if (p->d <= 64) return bf16 ? launch_fwd<true, 64, 0>(p, zero_pads, skip_single, s) : launch_fwd<false, 64, 0>(p, zero_pads, skip_single, s);
-  if (p->d <= 128) return bf16 ? launch_fwd<true, 128, 0>(p, zero_pads, skip_single, s) : launch_fwd<false, 128, 0>(p, zero_pads, skip_single, s);
-  return bf16 ? launch_fwd<true, 256, 0>(p, zero_pads, skip_single, s) : launch_fwd<false, 256, 0>(p, zero_pads, skip_single, s);
+  return go(launch_fwd<BF16, 128, FB, false>, launch_fwd<BF16, 128, FB, true>);
+}
+template <bool BF16>
+int launch_fwd_fb(const bsa_fwd_params* p, int zero_pads, int skip_single, cudaStream_t s) {
+  if (p->fine_block == 16) return launch_fwd_d<BF16, 16>(p, zero_pads, skip_single, s);
+  if (p->fine_block == 32) return launch_fwd_d<BF16, 32>(p, zero_pads, skip_single, s);
+  return launch_fwd_d<BF16, 0>(p, zero_pads, skip_single, s);
 }
 }  // namespace
 
@@ -859,7 +888,8 @@ int sm100_fwd(const bsa_fwd_params* pp, cudaStream_t s) {
   const int skip_single = p->total_q > 0 && p->q_start != p->k_start && p->total_q != p->sk && p->batch >= 4 &&
                           p->batch <= 65535 && p->causal && p->fine_block == 0 &&
                           p->row_mode == BSA_ROWS_BY_POSITION && (p->d == 64 || p->d == 128);
-  const int rc = launch_fwd_for(p, zero_pads, skip_single, s);
+  const int rc = p->dtype == BSA_BF16 ? launch_fwd_fb<true>(p, zero_pads, skip_single, s)
+                                      : launch_fwd_fb<false>(p, zero_pads, skip_single, s);
   return rc || !skip_single ? rc : decode_packed_rows(p, s);
 }
 

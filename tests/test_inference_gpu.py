@@ -660,6 +660,34 @@ def test_decode_weights_keep_their_fp32_value(fp8, Hq, Hkv, D, dtype):
     assert err <= 2e-5, float(err)
 
 
+@pytest.mark.parametrize("D,bs,dtype", [(64, 64, torch.bfloat16), (128, 64, torch.float16), (256, 64, torch.bfloat16),
+                                        (128, 32, torch.bfloat16), (64, 16, torch.float16)])
+def test_packed_batch_with_more_than_64k_keys_keeps_fp32_weights(D, bs, dtype):
+    """Such calls were computed in fp32 before the tensor cores took them.  Against 64 bits their error is the rounding
+    of the output and nothing else worth the name (5 %); 16-bit weights would add 40 % to it."""
+    Hq, Hkv, S, n_seq = 2, 1, 4096, 17
+    pk = dict(block_size=bs, local_blocks=256 // bs, vert_stride=5, num_kv_heads=Hkv)
+    mod = _module(Hq, S, pk, impl="sm100")
+    q_lens = [1 if i % 3 == 0 else 67 if i % 3 == 1 else 64 for i in range(n_seq)]
+    k_lens = [(3840 if n > 1 else 4000) + n for n in q_lens]          # chunks start on a block boundary
+    assert sum(k_lens) > 65536
+    q, k, v = (t.cuda() for t in seeded_qkv(103, (sum(q_lens), Hq, D), (sum(k_lens), Hkv, D), dtype))
+    cu_q, cu_k = (torch.tensor(np.cumsum([0] + n), dtype=torch.int32, device="cuda") for n in (q_lens, k_lens))
+    with torch.no_grad():
+        out = mod(q, k, v, cu_seqlen_k=cu_k, cu_seqlen_q=cu_q)
+    bm = torch.from_numpy(np.asarray(O.block_mask(Hq, S, **pk)).astype(bool)).cuda()
+    ref = torch.empty(out.shape, dtype=torch.float64, device="cuda")
+    for i, (nq, nk) in enumerate(zip(q_lens, k_lens)):
+        rows, keys = slice(int(cu_q[i]), int(cu_q[i + 1])), slice(int(cu_k[i]), int(cu_k[i + 1]))
+        qpos, kpos = torch.arange(nk - nq, nk, device="cuda"), torch.arange(nk, device="cuda")
+        for h in range(Hq):
+            on = bm[h % bm.size(0)][(qpos // bs)[:, None], (kpos // bs)[None]] & (kpos[None] <= qpos[:, None])
+            a = q[rows, h].double() @ k[keys, 0].double().T / math.sqrt(D)
+            ref[rows, h] = torch.softmax(a.masked_fill(~on, -math.inf), -1) @ v[keys, 0].double()
+    err, rounding = (out.double() - ref).norm(), (ref.to(dtype).double() - ref).norm()
+    assert err <= 1.05 * rounding, float(err / rounding)
+
+
 @pytest.mark.parametrize("many_keys", [False, True])
 @pytest.mark.parametrize("Hq,Hkv,D,bs,dtype", [(4, 2, 64, 32, torch.bfloat16), (3, 3, 128, 16, torch.float16),
                                                (2, 2, 64, 16, torch.bfloat16), (4, 1, 128, 32, torch.float16)])
