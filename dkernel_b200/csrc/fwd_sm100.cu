@@ -339,6 +339,9 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
     // items from it as they go (long tiles first, so the CTAs finish within one short tile of
     // each other); without one, round r hands items [r * grid, (r + 1) * grid) to the CTAs,
     // odd rounds in reverse CTA order so that no CTA collects the longest tile of every round.
+    // An item is drawn when there is a plan to fill, not before: drawn one earlier, a CTA held up to three
+    // tiles when the counter ran out (16 chunks of 256 tokens behind 1024: 88 -> 86 us; 19 prompts of up to
+    // 1766 tokens, a pattern per head: 193 -> 188 us).
     const bool wide = reinterpret_cast<uintptr_t>(p.o) % 16 == 0 && p.o_ss % 8 == 0 && p.o_sh % 8 == 0 &&
                       p.o_sb % 8 == 0;
     if (zero_pads) {
@@ -347,6 +350,8 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
       __syncwarp();
     }
     for (int k = 0;; ++k) {
+      const int pb = k & 1;
+      if (!mbar_wait(&tl->plan_free[pb], ((k >> 1) & 1) ^ 1, wait_status, 401)) break;
       int item;
       if (p.tile_counter) {
         item = 0;
@@ -356,8 +361,6 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
         const long long it = (long long)k * gridDim.x + ((k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
         item = it < n_items ? (int)it : n_items;
       }
-      const int pb = k & 1;
-      if (!mbar_wait(&tl->plan_free[pb], ((k >> 1) & 1) ^ 1, wait_status, 401)) break;
       if (item >= n_items || item < 0 ||
           !build_plan<FB>(p, mode, item, tiles_x, head_items, skip_single, &tl->plan[pb], tl->bits, lane, wait_status)) {
         if (lane == 0) {
