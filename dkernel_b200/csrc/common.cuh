@@ -84,6 +84,7 @@ int sm100_bwd(const bsa_bwd_params* p, cudaStream_t s);
 size_t decode_workspace_bytes(const bsa_decode_params* p);
 int decode_run(const bsa_decode_params* p, cudaStream_t s);
 int decode_packed_rows(const bsa_fwd_params* p, cudaStream_t s);
+constexpr int kMaxRowBlocks = 1024;   // 64-token blocks that a prefill tile or a packed decode row can list
 int decode_run_static(const bsa_decode_params* p, cudaStream_t s);
 size_t decode_static_capacity();
 int merge_partials(const void* o_parts, const float* lse_parts, int P, int64_t rows, int d,

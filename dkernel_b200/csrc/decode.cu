@@ -34,7 +34,6 @@ constexpr int kMinCtas = 3;              // resident CTAs per SM the kernel is b
 constexpr int kConsumers = 4;            // consumer warps
 constexpr int kDecThreads = 32 * (kConsumers + 1);
 constexpr int kMaxTokens = 4096;         // tokens per CTA (a caller's blocks_per_split)
-constexpr int kMaxRowBlocks = 1024;      // blocks of one row in a packed batch (decode_packed_rows)
 constexpr float kDecRescale = 8.0f;      // log2 of how far a maximum may grow before O is rescaled
 
 constexpr int kClusterCtas = 128;        // CTAs per resident CTA of an SM up to which a grid runs as clusters
@@ -197,6 +196,8 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
 // heads, D 128, local 16 + stride 8, with the merge kernel: 68 us for the 401 MB of a bf16 cache, 53 us for
 // the 203 MB of an e4m3 cache (67.5 and 52.4 with P in one term).  (78 and 79 us when all four warps shared a unit, 16 tokens each, with the
 // heads on the rows; 71 and 56 us when a producer warp refilled K and V together after both were read.)
+// Nine to 16 heads, 2 kv heads, D 128, the same sequences: 27 to 30 us bf16 (heads on the rows: 26 to 29),
+// 29 to 31.5 e4m3 (30 to 32); D 64 18 to 19 us (19 to 21).
 template <typename T, int D, bool FP8, int NT, bool FOLD>
 __global__ void __launch_bounds__(kDecThreads, FP8 && D == 128 && NT == 2 ? 2 : kMinCtas)   // 2: spills otherwise
 decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 tmV,
@@ -926,7 +927,9 @@ int decode_run(const bsa_decode_params* p, cudaStream_t s) {
   // CTAs merge their parts over distributed shared memory: no partials and no second launch.  In a larger
   // grid waiting for a cluster's worth of room costs more than the second launch.  (Sequences of 3000 to 4096
   // tokens, 32/8 heads, D 128, 64 CTAs each: 1: 13.3 -> 11.3 us, 2: 13.3 -> 11.9, 4: 14.0 -> 13.3, 6: 15.4 ->
-  // 13.3, 8: 17.1 -> 21.5 us; 64 of 1024 to 8192 tokens: 69 -> 71 us.)
+  // 13.3, 8: 17.1 -> 21.5 us; 64 of 1024 to 8192 tokens: 69 -> 71 us.  Those are eight splits; two to seven,
+  // one sequence and as many as the limit takes: 2: 8.5 -> 7.8, 24: 12.2 -> 10.0; 4: 9.4 -> 8.2, 12: 12.8 -> 10.5;
+  // 7: 10.3 -> 8.7, 6: 12.8 -> 11.0 us; e4m3 the same.)
   const long long ctas = (long long)p->batch * (p->hq / p->heads_per_cta) * nsplit;
   const int resident = fp8 && p->d == 128 && p->heads_per_cta > 8 ? 2 : kMinCtas;   // the kernel's launch bounds
   const int cl = p->o && nsplit > 1 && nsplit <= kMaxCluster && ctas <= kClusterCtas * resident ? nsplit : 1;
@@ -935,13 +938,10 @@ int decode_run(const bsa_decode_params* p, cudaStream_t s) {
 }
 
 // The sequences of a packed batch that have one query token.  A CTA walks a whole pattern row (there
-// is no scratch for partials); its list holds every block of the pattern's longest possible row.  (Two or
-// four CTAs per row as a cluster: 163 and 221 us for the batch of sm100_fwd's comment, against 135.)
+// is no scratch for partials); its list holds every block of the pattern's longest possible row, which is
+// kMaxRowBlocks at most (sm100_fwd_supported: rows or keys of the call are bounded by it).  (Two or four CTAs
+// per row as a cluster: 163 and 221 us for the batch of sm100_fwd's comment, against 135 at the time.)
 int decode_packed_rows(const bsa_fwd_params* f, cudaStream_t s) {
-  if (f->n_rows > kMaxRowBlocks && f->sk > kMaxRowBlocks * 64) {
-    set_error("bsa_fwd: a row of a packed batch has more than %d blocks", kMaxRowBlocks);
-    return BSA_E_TOOBIG;
-  }
   bsa_decode_params p = {};
   p.q = f->q; p.k = f->k; p.v = f->v; p.o = f->o; p.lse = f->lse;
   p.q_sb = f->q_ss; p.q_sh = f->q_sh;

@@ -26,7 +26,7 @@ namespace {
 constexpr int kBS = 64;
 constexpr int kThreadsP = 224;
 constexpr int kWarpProd = 4, kWarpIssue = 5, kWarpPlan = 6;
-constexpr int kMaxList = 1024;           // kv blocks per sequence (64K tokens)
+constexpr int kMaxList = kMaxRowBlocks;  // kv blocks per sequence (64K tokens)
 constexpr uint32_t kBlkMask = kMaxList - 1;   // the block of a list entry
 // Shared-memory tiles are stored as D/64 sub-tiles of [rows][128 bytes] (one TMA box each,
 // 128-byte swizzled): Q 128 rows (16 KB per sub-tile), K and V 64 rows (8 KB per sub-tile).
@@ -795,7 +795,7 @@ bool sm100_fwd_supported(const bsa_fwd_params* p, const char** why) {
   // together (a serving step with 48 contexts has hundreds of thousands); what bounds one sequence's
   // list there is the pattern: under the causal mask a row lists no block past its own index.
   // (3 chunks of 512 tokens + 45 decode tokens over 192 thousand keys, 32/8 heads, D 128: 12.6 ms
-  // on the CUDA-core kernel, 0.21 ms here.)
+  // on the CUDA-core kernel, 0.145 ms here.)
   const bool packed_rows = p->total_q > 0 && p->causal && p->row_mode == BSA_ROWS_BY_POSITION && p->n_rows <= kMaxList;
   if (p->sk > kMaxList * kBS && !packed_rows) return no("more than 65536 key positions");
   if (!tma_compatible(p->q, 2, p->q_ss, p->q_sh, p->q_sb) ||
@@ -883,7 +883,8 @@ int sm100_fwd(const bsa_fwd_params* pp, cudaStream_t s) {
   // prompts does not pass): sequences with one query token go to the decode kernel, which reads their
   // K/V once for all heads of a group instead of walking them in 64-row tiles with one row in use.
   // 3 chunks of 512 tokens and 45 decode tokens over 192 thousand keys, 32/8 heads, D 128: 197 us with
-  // all of them as tiles, 147 us with the decode kernel in front of this one, 130 us behind it.
+  // all of them as tiles, 147 us with the decode kernel in front of this one, 130 us behind it (weights in
+  // one 16-bit term; 145 us as it is, see SPLIT).
   // How many there are stands on the device only, and where there are none the launch costs 0.6 to 1 us
   // for nothing.  So not where as many queries as keys say whole prompts, nor below four sequences, where
   // it is a tenth of a small call (a chunk of 64: 8.5 -> 9.3 us) and one to three tokens fit beside the

@@ -220,8 +220,9 @@ int bsa_bwd(const bsa_bwd_params* p, void* stream);
  * (dkernel/ops/sparse_attn_inference.py:83-88, :141) and the sliced-crow decode
  * of _forward (dkernel/ops/sparse_attn_fwd.py:435-440).  Split-KV: every
  * (sequence, kv head, split) is one CTA; the partial (O, m, l) of small grids are
- * merged inside the launch, others go to the workspace and are merged by a second
- * kernel.
+ * merged inside the launch (the workspace is asked for all the same, but not
+ * touched), others go to the workspace and are merged by a second kernel.
+ * Any sm_scale is served, negative ones and 0 as well.
  * ------------------------------------------------------------------------- */
 typedef struct {
   const void* q;              /* (batch, hq, d), strides q_sb, q_sh             */
