@@ -75,11 +75,6 @@ template <> struct MmaType<__half> {
     __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
   }
-  // what the packed pair leaves of its two sources
-  static __device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t packed) {
-    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&packed));
-    return pack(lo - h.x, hi - h.y);
-  }
 };
 template <> struct MmaType<__nv_bfloat16> {
   static __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
@@ -93,9 +88,6 @@ template <> struct MmaType<__nv_bfloat16> {
   static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
-  }
-  static __device__ __forceinline__ uint32_t pack_rest(float lo, float hi, uint32_t packed) {
-    return pack(lo - __uint_as_float(packed << 16), hi - __uint_as_float(packed & 0xffff0000u));
   }
 };
 
@@ -130,7 +122,7 @@ __device__ __forceinline__ float dec_ex2(float x) {
 // the V reads below free of bank conflicts); the consumer warps read the stored bytes with plain
 // 16-byte loads and convert them straight into tensor-core fragments in registers.  e4m3 converts
 // to f16 exactly and in one instruction per pair, so with an 8-bit cache the products run in f16
-// whatever the type of q (q is converted once while it is staged; P lies in [0, 2^kDecRescale]).
+// whatever the type of q (q is converted once while it is staged; P lies in [0, 2^15]).
 //
 // Fragment trick of the 8-bit path: a product's contraction index may be enumerated in any order,
 // and so may the output rows, as long as both operands (resp. the epilogue) agree.
@@ -183,10 +175,10 @@ __device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s
 
 // NT: 8-column tiles of q heads (heads_per_cta <= 8 NT).
 //
-// P enters V^T P^T as two 16-bit terms, P = hi + lo, which keeps its fp32 value to 2^-16 (bf16) or better.
+// P enters V^T P^T as two 16-bit terms, P = hi + lo (two_terms), which keeps its fp32 value to 2^-16 (bf16) or better.
 // One term rounds every weight at 2^-9 (bf16) or 2^-12 (f16), and a reference maximum that is raised lazily
 // leaves not even a row's largest weights exact: error against 64 bits, apart from the rounding of the output,
-// 1.53e-3 of the output with bf16 and 1.8e-4 with e4m3 K/V, now 2.4e-6 and 2.5e-7.  FOLD: where the last
+// 1.53e-3 of the output with bf16 and 1.8e-4 with e4m3 K/V, now 4.6e-6 and 2.8e-7.  FOLD: where the last
 // tile holds up to four heads, their lo terms take its columns 4..7 (its q rows 4..7 repeat rows 0..3, so that
 // the logits are there already) and cost no product of their own (the e4m3 step below 53.0 instead of 55.7 us);
 // those of a fuller tile are a second product on the same V fragments.
@@ -213,6 +205,8 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
                                              ~uintptr_t(1023));
   uint8_t* ring = smem;
   using MT = typename std::conditional<FP8, __half, T>::type;   // type of the tensor-core products
+  constexpr bool kBf16 = std::is_same<MT, __nv_bfloat16>::value;
+  constexpr float kShift = kTermShift<kBf16>;
   auto* sm = reinterpret_cast<DecodeSmem<D, FP8, NT>*>(smem + kRingBytes);
 
   // the merge kernel behind this one may be made resident as soon as every CTA got here
@@ -511,15 +505,17 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
       uint32_t pb[kTok / 16][NT][2], pl[kTok / 16][NT][2];
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        const float n0 = m[nt][0] == -INFINITY ? 0.f : -m[nt][0], n1 = m[nt][1] == -INFINITY ? 0.f : -m[nt][1];
+        const float n0 = m[nt][0] == -INFINITY ? 0.f : kShift == 0.f ? -m[nt][0] : kShift - m[nt][0];
+        const float n1 = m[nt][1] == -INFINITY ? 0.f : kShift == 0.f ? -m[nt][1] : kShift - m[nt][1];
 #pragma unroll
         for (int mt = 0; mt < kTok / 16; ++mt) {
           const float p0 = dec_ex2(fmaf(sacc[mt][nt][0], mul, n0)), p1 = dec_ex2(fmaf(sacc[mt][nt][1], mul, n1));
           const float p2 = dec_ex2(fmaf(sacc[mt][nt][2], mul, n0)), p3 = dec_ex2(fmaf(sacc[mt][nt][3], mul, n1));
           l[nt][0] += p0 + p2;
           l[nt][1] += p1 + p3;
-          const uint32_t hi0 = MmaType<MT>::pack(p0, p1), hi1 = MmaType<MT>::pack(p2, p3);
-          const uint32_t lo0 = MmaType<MT>::pack_rest(p0, p1, hi0), lo1 = MmaType<MT>::pack_rest(p2, p3, hi1);
+          uint32_t hi0, lo0, hi1, lo1;
+          two_terms<kBf16, !FP8>(p0, p1, hi0, lo0);
+          two_terms<kBf16, !FP8>(p2, p3, hi1, lo1);
           pb[mt][nt][0] = transpose8x8(FOLD && nt == NT - 1 && tq >= 2 ? lo0 : hi0);
           pb[mt][nt][1] = transpose8x8(FOLD && nt == NT - 1 && tq >= 2 ? lo1 : hi1);
           if (nt < kLoTiles) {
@@ -596,7 +592,7 @@ decode_kernel(const __grid_constant__ Tmap4 tmK, const __grid_constant__ Tmap4 t
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) l[nt][e] += __shfl_xor_sync(0xffffffffu, l[nt][e], o);
         if (g == 0) {
-          sm->wm[warp][nt * 8 + 2 * tq + e] = m[nt][e];
+          sm->wm[warp][nt * 8 + 2 * tq + e] = m[nt][e] - kShift;   // the maximum that O and l are relative to
           sm->wl[warp][nt * 8 + 2 * tq + e] = l[nt][e];
         }
       }

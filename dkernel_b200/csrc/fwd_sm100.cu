@@ -91,21 +91,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
-// what the 16-bit pair `hi` leaves of lo, hi's sources: the second term of P = P_hi + P_lo
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2_rest(float p0, float p1, uint32_t hi) {
-  float h0, h1;
-  if (BF16) {
-    h0 = __uint_as_float(hi << 16);
-    h1 = __uint_as_float(hi & 0xffff0000u);
-  } else {
-    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-    h0 = h.x;
-    h1 = h.y;
-  }
-  return pack2<BF16>(p0 - h0, p1 - h1);
-}
-
 // item -> plan (executed by the whole planner warp)
 // Returns false when no sequence has this tile, nor any tile of a later item.
 template <int FB>
@@ -282,9 +267,9 @@ __device__ __forceinline__ void store_pad_rows(const bsa_fwd_params& p, int head
 // FB: 0, or the pattern's own block size (16 or 32) when it is finer than the 64-token tiles: the
 // CSR then describes the pattern coarsened to 64 x 64 blocks and col_bits holds, per CSR entry,
 // one bit per (sub-row, sub-column) pair of the block (bit a * (64/FB) + b).
-// SPLIT: P = hi + lo, two 16-bit terms side by side in S's columns and 128 instead of 64 "tokens" for
+// SPLIT: P = hi + lo (two_terms), two 16-bit terms side by side in S's columns and 128 instead of 64 "tokens" for
 // P V, the second half on the same V rows.  Error against 64 bits apart from the rounding of the output,
-// chunks beside decode tokens, bf16: 1.6e-3 of the output with one term, 4e-6 with two (fp32 arithmetic on
+// chunks beside decode tokens, bf16: 1.6e-3 of the output with one term, 6e-6 with two (fp32 arithmetic on
 // the CUDA cores: 7e-7); the call as a whole 130 -> 145 us (12.6 ms there).
 template <bool BF16, int D, int FB, bool SPLIT>
 __global__ void __launch_bounds__(kThreadsP, D <= 128 ? 2 : 1)
@@ -520,6 +505,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
     const int rr = r & 63;
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
     const float scale2 = p.sm_scale * kLog2e;
+    constexpr float kShift = SPLIT ? kTermShift<BF16> : 0.f;
     const bool wide = reinterpret_cast<uintptr_t>(p.o) % 16 == 0 && p.o_ss % 8 == 0 &&
                       p.o_sh % 8 == 0 && p.o_sb % 8 == 0;   // rows start on 16-byte boundaries
     uint32_t g = 0;      // kv blocks processed so far, over all tiles
@@ -655,7 +641,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
         // P is produced and stored in two halves, so that the first store's latency is covered
         // by the second half's exponentials and fewer packed values are live at a time
         const bool live = att && m_used != -INFINITY;
-        const float neg_m = -m_used;
+        const float neg_m = kShift == 0.f ? -m_used : kShift - m_used;
         // two columns per fused multiply-add and per addition (packed fp32 pairs): the softmax
         // warps are bound by instruction issue as much as by the exponential unit
         const uint64_t scale_2 = f32x2(scale2, scale2), neg_m2 = f32x2(neg_m, neg_m);
@@ -670,8 +656,8 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
               f32x2_split(fma_f32x2(f32x2(sv[hlf * 32 + 2 * c], sv[hlf * 32 + 2 * c + 1]), scale_2, neg_m2), x0, x1);
               const float p0 = ex2(x0), p1 = ex2(x1);
               sum2[c & 1] = add_f32x2(sum2[c & 1], f32x2(p0, p1));
-              pk[c] = pack2<BF16>(p0, p1);
-              if (SPLIT) pl[SPLIT ? c : 0] = pack2_rest<BF16>(p0, p1, pk[c]);
+              if constexpr (SPLIT) two_terms<BF16, true>(p0, p1, pk[c], pl[c]);
+              else pk[c] = pack2<BF16>(p0, p1);
             }
           } else {
 #pragma unroll
@@ -768,7 +754,7 @@ fwd_persist_kernel(const __grid_constant__ Tmap4 tmQ, const __grid_constant__ Tm
               *reinterpret_cast<uint2*>(orow + ch * 64 + i * 8) = make_uint2(w[2 * i], w[2 * i + 1]);
         }
       }
-      if (row_ok && lse_ptr) *lse_ptr = l > 0.f ? (m_used + log2f(l)) * kLn2 : -INFINITY;
+      if (row_ok && lse_ptr) *lse_ptr = l > 0.f ? (m_used - kShift + log2f(l)) * kLn2 : -INFINITY;
       __syncwarp();
       if (lane == 0) mbar_arrive(&tl->plan_free[pb]);
       ++k;

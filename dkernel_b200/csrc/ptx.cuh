@@ -116,6 +116,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
+// Weights 2^x as two 16-bit terms, p = hi + lo: hi cut off, lo what it leaves (rounded: 2^-16 of p or less).
+// Where p > 0 both terms are, so that an infinity in V stays one (0 * inf would be NaN): lo is at least 2^-18 p in
+// bf16.  f16 has no room for that below 1, so its x comes raised by kTermShift (2^15 at most when the reference
+// maximum lags 2^8 behind), and lo is at least the smallest f16, 2^-31 of a weight at the reference.
+// INF = false: V's type has no infinity.
+template <bool BF16> constexpr float kTermShift = BF16 ? 0.f : 7.f;
+template <bool BF16, bool INF>
+__device__ __forceinline__ void two_terms(float p0, float p1, uint32_t& hi, uint32_t& lo) {
+  float h0, h1;
+  if (BF16) {
+    asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(hi) : "r"(__float_as_uint(p0)), "r"(__float_as_uint(p1)));
+    h0 = __uint_as_float(hi << 16);
+    h1 = __uint_as_float(hi & 0xffff0000u);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(fmaxf(p0 - h0, p0 * 0x1p-18f), fmaxf(p1 - h1, p1 * 0x1p-18f));
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  } else {
+    asm("cvt.rz.f16x2.f32 %0, %2, %1;" : "=r"(hi) : "f"(p0), "f"(p1));
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    const __half2 l = __floats2half2_rn(INF && p0 > 0.f ? fmaxf(p0 - h.x, 0x1p-24f) : p0 - h.x,
+                                        INF && p1 > 0.f ? fmaxf(p1 - h.y, 0x1p-24f) : p1 - h.y);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  }
+}
+
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

@@ -709,3 +709,44 @@ def test_packed_fine_blocks_from_any_position(Hq, Hkv, D, bs, dtype, many_keys):
         out, lse = mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda(), return_lse=True)
     assert_out_close(out, ref)
     assert_lse_close(lse, ref_lse)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Hq,Hkv,D", [(4, 1, 128), (8, 1, 64), (12, 1, 128), (16, 1, 64)])
+def test_decode_leaves_an_infinity_in_v_one(Hq, Hkv, D, dtype):
+    """+-inf in V gives +-inf in that column of the output, not NaN: no term of a weight above 0 may be 0 (q of zeros:
+    equal weights, exact in 16 bits) or have the other sign; the other columns are not touched."""
+    bs, S, lens = 64, 512, [512, 100, 64]
+    pk = dict(block_size=bs, local_blocks=8, vert_stride=4, num_kv_heads=Hkv)
+    q, k, v = seeded_qkv(109, (3, 1, Hq, D), (3, S, Hkv, D), dtype)
+    q[2] = 0
+    left = torch.tensor([S - n for n in lens], dtype=torch.int32)
+    ref, _ = O.decode_attention(q.float(), k.float(), v.float(), O.block_mask(Hq, S, **pk), bs, left_paddings=left)
+    v[:, S - 50, :, 3], v[:, S - 7, :, D - 1] = float("inf"), float("-inf")
+    with torch.no_grad():
+        out = _module(Hq, S, pk, seq_dim=1)(q.cuda(), k.cuda(), v.cuda(), left_paddings=left.cuda()).cpu()
+    assert (out[..., 3] == float("inf")).all() and (out[..., D - 1] == float("-inf")).all()
+    keep = [c for c in range(D) if c not in (3, D - 1)]
+    assert_out_close(out[..., keep], ref[..., keep])
+
+
+@pytest.mark.parametrize("D,bs,dtype", [(64, 64, torch.bfloat16), (128, 64, torch.float16), (64, 32, torch.float16)])
+def test_packed_batch_with_more_than_64k_keys_leaves_an_infinity_in_v_one(D, bs, dtype):
+    Hq, Hkv, S, n_seq = 2, 1, 4096, 17
+    pk = dict(block_size=bs, local_blocks=256 // bs, vert_stride=5, num_kv_heads=Hkv)
+    q_lens = [1 if i % 3 == 0 else 67 for i in range(n_seq)]
+    k_lens = [3840 + n for n in q_lens]
+    cu_q, cu_k = (torch.tensor(np.cumsum([0] + n), dtype=torch.int32) for n in (q_lens, k_lens))
+    q, k, v = seeded_qkv(111, (sum(q_lens), Hq, D), (sum(k_lens), Hkv, D), dtype)
+    q[:40] = 0
+    mod = _module(Hq, S, pk, impl="sm100")
+
+    def call():
+        with torch.no_grad():
+            return mod(q.cuda(), k.cuda(), v.cuda(), cu_seqlen_k=cu_k.cuda(), cu_seqlen_q=cu_q.cuda()).cpu()
+    ref = call()
+    first = cu_k[:-1].long() + 3840             # every query of a sequence attends its first one's key
+    v[first, :, 3], v[first, :, D - 1] = float("inf"), float("-inf")
+    out = call()
+    assert (out[..., 3] == float("inf")).all() and (out[..., D - 1] == float("-inf")).all()
+    assert torch.equal(out[..., 4:D - 1], ref[..., 4:D - 1])
